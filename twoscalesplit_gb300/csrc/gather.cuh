@@ -3,10 +3,8 @@
 // PerThread: one particle per thread, 32 particles per warp.  Each thread walks its
 // window's rows in order, testing each candidate and evaluating an accepted pair
 // at once.  This is the throughput form: consecutive threads walk overlapping
-// windows, so neighbour loads are shared through L1.  (A cursor that searched on
-// to the next accepted candidate before evaluating, so that a warp's lanes met at
-// the pair arithmetic, was 4-8 % slower in the density gathers and no faster in
-// the force gathers on a developed 1M-particle dam break.)
+// windows, so neighbour loads are shared through L1.  The same-scale sums, which
+// are most of the work, are taken from lists instead (nbr_search, gathers.cuh).
 //
 // PerWarp: one particle per warp.  The 32 lanes test 32 consecutive candidates of
 // a row at a time and evaluate the accepted pairs' terms in parallel; then every
@@ -54,40 +52,20 @@ struct PerThread {
     }
 
     // window() for a walk whose test is a key of the candidate alone: key(k) (a
-    // float, e.g. the squared distance), ok(x) the test on it, term(k, x).  U (2 or
-    // 4) candidates per trip: their keys are formed before any of their terms is
-    // evaluated, in candidate order, which cuts the loop's own instructions and
-    // keeps U neighbour loads in flight.  On a developed 1M-particle dam break, two
-    // per trip took 3-7 % off the densities against one; four took 4-5 % more off
-    // the high-res density (whose key also loads the candidate's state) and was
-    // 2-3 % slower than two in the low-res density.
-    template <int U, class T, class Key, class Ok, class Term, class Add>
+    // float, e.g. the squared distance), ok(x) the test on it, term(k, x).  The
+    // per-thread densities search and evaluate apart (nbr_search, gathers.cuh) and
+    // come here only with the particles that does not take.
+    template <class T, class Key, class Ok, class Term, class Add>
     __device__ __forceinline__ static void window_keyed(const int* off, int dimx, int csx, int cex, int csy, int cey,
                                                         Key&& key, Ok&& ok, Term&& term, Add&& add, T& sum) {
-        static_assert(U == 2 || U == 4, "two or four candidates per trip");
-        for (int cy = csy; cy <= cey; ++cy) {
-            const int row = cy * dimx;
-            const int b = off[row + cex + 1];
-            int k = off[row + csx];
-            if constexpr (U == 4) {
-                for (; k + 3 < b; k += 4) {
-                    const float x0 = key(k), x1 = key(k + 1), x2 = key(k + 2), x3 = key(k + 3);
-                    if (ok(x0)) add(sum, term(k, x0));
-                    if (ok(x1)) add(sum, term(k + 1, x1));
-                    if (ok(x2)) add(sum, term(k + 2, x2));
-                    if (ok(x3)) add(sum, term(k + 3, x3));
-                }
-            }
-            for (; k + 1 < b; k += 2) {
-                const float x0 = key(k), x1 = key(k + 1);
-                if (ok(x0)) add(sum, term(k, x0));
-                if (ok(x1)) add(sum, term(k + 1, x1));
-            }
-            if (k < b) {
-                const float x0 = key(k);
-                if (ok(x0)) add(sum, term(k, x0));
-            }
-        }
+        float x = 0.0f;
+        window(
+            off, dimx, csx, cex, csy, cey,
+            [&](int k) {
+                x = key(k);
+                return ok(x);
+            },
+            [&](int k) { return term(k, x); }, add, sum);
     }
 
     // window() over the rows for which live(row) holds (row = cy * dimx).  A row
@@ -133,7 +111,7 @@ struct PerWarp {
         }
     }
 
-    template <int U, class T, class Key, class Ok, class Term, class Add>
+    template <class T, class Key, class Ok, class Term, class Add>
     __device__ __forceinline__ static void window_keyed(const int* off, int dimx, int csx, int cex, int csy, int cey,
                                                         Key&& key, Ok&& ok, Term&& term, Add&& add, T& sum) {
         float x = 0.0f;

@@ -60,32 +60,86 @@ using namespace gather_detail;
 // particle with more than kMaxNbr neighbours, or one whose offset does not fit
 // 16 bits, is marked and walks its window.
 //
-// The entries are staged in shared memory as they are found (`col`: the thread's
-// column of a kMaxNbr x kNbrCols array, stride kNbrCols) and written out after the
-// walk, entry c of every lane together, so that a warp's stores to the transposed
-// global array coalesce; stored as found, they scattered over its rows.
-constexpr int kNbrCols = 256;  // the gathers' largest block
+// The density pass takes a particle's same-scale window in two phases.  The first
+// walks the window and only tests: it leaves the accepted candidates' offsets in
+// shared memory (`col`: the thread's column of a kNbrRows x kNbrCols array, stride
+// kNbrCols), a few instructions per candidate.  The second walks that short list,
+// evaluates the pairs' terms in order and writes the list out.  A warp's lanes
+// accept different candidates of the ~34 in their windows, so a walk that evaluates
+// a pair as soon as its test passes runs the pair arithmetic for nearly every
+// candidate with a third of the lanes active; here it runs once per list entry with
+// almost all of them (the lists are 10-14 long).
+constexpr int kNbrCols = 256;          // the gathers' largest block
+constexpr int kNbrRows = kMaxNbr + 5;  // the particle itself, and one trip of four past a full list
 
-struct NbrRecord {
-    int16_t* col;
-    int i, n;
-    bool ok;
-    __device__ __forceinline__ NbrRecord(int i_, int16_t* col_) : col(col_), i(i_), n(0), ok(true) {}
-    __device__ __forceinline__ void add(int j) {
-        if (j == i) return;  // the density's self term: never a force pair
-        const int dj = j - i;
-        if (n < kMaxNbr && dj >= -32768 && dj <= 32767) col[n * kNbrCols] = static_cast<int16_t>(dj);
-        else ok = false;
-        ++n;
-    }
-    __device__ __forceinline__ void finish(const ScaleView& S) const {
-        if (ok) {
-            int16_t* dst = S.nbr + i;  // 64-bit steps: a pool's capacity times kMaxNbr passes 2^31
-            for (int c = 0; c < n; ++c, dst += S.nbr_stride) *dst = col[c * kNbrCols];
+// Phase one: the candidates k of the window with key(k) <= T (a NaN key fails), in
+// window order, as k - i in the column.  Returns their number, or -1 when there are
+// more than the list holds or an offset does not fit 16 bits.
+template <class Key>
+__device__ __forceinline__ int nbr_search(const int* off, int dimx, int csx, int cex, int csy, int cey, int i, float T,
+                                          int16_t* col, Key&& key) {
+    int16_t* c = col;
+    int16_t* const full = col + (kMaxNbr + 1) * kNbrCols;
+    const auto put = [&](int k, float x) {
+        if (x <= T) {
+            *c = static_cast<int16_t>(k - i);
+            c += kNbrCols;
         }
-        S.nnbr[i] = ok ? static_cast<uint8_t>(n) : kNbrOverflow;
+    };
+    for (int cy = csy; cy <= cey; ++cy) {
+        const int row = cy * dimx;
+        int k = off[row + csx];
+        const int b = off[row + cex + 1];
+        if (k - i < -32768 || b - i > 32768) return -1;
+        for (; k + 3 < b; k += 4) {
+            const float x0 = key(k), x1 = key(k + 1), x2 = key(k + 2), x3 = key(k + 3);
+            put(k, x0);
+            put(k + 1, x1);
+            put(k + 2, x2);
+            put(k + 3, x3);
+            if (c > full) return -1;
+        }
+        if (k + 1 < b) {
+            const float x0 = key(k), x1 = key(k + 1);
+            put(k, x0);
+            put(k + 1, x1);
+            k += 2;
+        }
+        if (k < b) put(k, key(k));
+        if (c > full) return -1;
     }
-};
+    return static_cast<int>(c - col) / kNbrCols;
+}
+
+// Phase two: adds the terms of the n entries in the column to `sum`, in order, and
+// writes the entries other than the particle itself to its neighbour list.
+template <class A>
+__device__ __forceinline__ void nbr_density(const Params& P, const ScaleView& S, int i, float2 p, int n,
+                                            const int16_t* col, float& sum) {
+    int16_t* const first = S.nbr + i;  // 64-bit steps: a pool's capacity times kMaxNbr passes 2^31
+    int16_t* dst = first;
+    int m = 0;
+    const auto entry = [&](int dj, float x) {
+        sum += A::density(P, x);
+        if (dj != 0) {
+            *dst = static_cast<int16_t>(dj);
+            dst += S.nbr_stride;
+            ++m;
+        }
+    };
+    int c = 0;
+    for (; c + 1 < n; c += 2) {
+        const int d0 = col[c * kNbrCols], d1 = col[(c + 1) * kNbrCols];
+        const float x0 = sq(sub(p, S.pos[i + d0])), x1 = sq(sub(p, S.pos[i + d1]));
+        entry(d0, x0);
+        entry(d1, x1);
+    }
+    if (c < n) {
+        const int d0 = col[c * kNbrCols];
+        entry(d0, sq(sub(p, S.pos[i + d0])));
+    }
+    S.nnbr[i] = static_cast<uint8_t>(m);
+}
 
 // A same-scale neighbour's state as the force pass reads it.
 struct NbrState {
@@ -150,22 +204,25 @@ __device__ __forceinline__ void density_high_one(const Params& P, const StepView
     float d = 0.0f, dl = 0.0f;
     float x = 0.0f;
     const auto term = [&](int) { return A::density(P, x); };
-    const bool rec_on = !G::kWarp && H.nbr != nullptr;
-    NbrRecord rec(i, nbr_col);
     int csx, csy, cex, cey;
     grid_coord_s<1>(P, p.x, p.y, -P.rh, csx, csy);
     grid_coord_s<1>(P, p.x, p.y, P.rh, cex, cey);
     // a candidate the lambda mask rejects gets key +inf: no cutoff passes it
-    G::template window_keyed<4>(
-        offH, P.dimH[0], csx, cex, csy, cey,
-        [&](int k) { return lamHH(s, H.st[k]) ? sq(sub(p, H.pos[k])) : INFINITY; },
-        [&](float xk) { return xk <= P.Tle_rh; },
-        [&](int j, float xj) {
-            if (rec_on) rec.add(j);
-            return A::density(P, xj);
-        },
-        add_density, d);
-    if (rec_on) rec.finish(H);
+    const auto masked = [&](int k) { return lamHH(s, H.st[k]) ? sq(sub(p, H.pos[k])) : INFINITY; };
+    int nn = -1;
+    if constexpr (!G::kWarp) {
+        if (s & 1u)  // the mask passes every candidate of a state-1 particle
+            nn = nbr_search(offH, P.dimH[0], csx, cex, csy, cey, i, P.Tle_rh, nbr_col,
+                            [&](int k) { return sq(sub(p, H.pos[k])); });
+        else
+            nn = nbr_search(offH, P.dimH[0], csx, cex, csy, cey, i, P.Tle_rh, nbr_col, masked);
+        if (nn >= 0) nbr_density<A>(P, H, i, p, nn, nbr_col, d);
+        else H.nnbr[i] = kNbrOverflow;
+    }
+    if (nn < 0)
+        G::window_keyed(
+            offH, P.dimH[0], csx, cex, csy, cey, masked, [&](float xk) { return xk <= P.Tle_rh; },
+            [&](int, float xj) { return A::density(P, xj); }, add_density, d);
     grid_coord_s<0>(P, p.x, p.y, -P.r, csx, csy);
     grid_coord_s<0>(P, p.x, p.y, P.r, cex, cey);
     // With no high-res entry in state 0 in this step (hstate0 false), a state-1
@@ -239,7 +296,7 @@ __device__ __forceinline__ void density_high_one(const Params& P, const StepView
 
 template <bool B, class G, class A>
 __global__ void __launch_bounds__(256) k_density_high(Params P0, StepView V) {
-    __shared__ int16_t s_nbr[G::kWarp ? 1 : kMaxNbr * kNbrCols];
+    __shared__ int16_t s_nbr[G::kWarp ? 1 : kNbrRows * kNbrCols];
     int16_t* const nbr_col = s_nbr + (G::kWarp ? 0 : threadIdx.x);
     const bool hstate0 = V.cnt->h_state0 != 0;
     for_each_particle<G>(V.cnt->cur[1], [&](int i) {
@@ -265,20 +322,20 @@ __device__ __forceinline__ void density_low_one(const Params& P, const StepView&
     float d = 0.0f, dh = 0.0f;
     float x = 0.0f;
     const auto term = [&](int) { return A::density(P, x); };
-    const bool rec_on = !G::kWarp && L.nbr != nullptr;
-    NbrRecord rec(i, nbr_col);
     int csx, csy, cex, cey;
     grid_coord_s<0>(P, p.x, p.y, -P.r, csx, csy);
     grid_coord_s<0>(P, p.x, p.y, P.r, cex, cey);
-    G::template window_keyed<2>(
-        L.off + P.cbL, P.dimL[0], csx, cex, csy, cey, [&](int k) { return sq(sub(p, L.pos[k])); },
-        [&](float xk) { return xk <= P.Tle_r; },
-        [&](int j, float xj) {
-            if (rec_on) rec.add(j);
-            return A::density(P, xj);
-        },
-        add_density, d);
-    if (rec_on) rec.finish(L);
+    const auto key = [&](int k) { return sq(sub(p, L.pos[k])); };
+    int nn = -1;
+    if constexpr (!G::kWarp) {
+        nn = nbr_search(L.off + P.cbL, P.dimL[0], csx, cex, csy, cey, i, P.Tle_r, nbr_col, key);
+        if (nn >= 0) nbr_density<A>(P, L, i, p, nn, nbr_col, d);
+        else L.nnbr[i] = kNbrOverflow;
+    }
+    if (nn < 0)
+        G::window_keyed(
+            L.off + P.cbL, P.dimL[0], csx, cex, csy, cey, key, [&](float xk) { return xk <= P.Tle_r; },
+            [&](int, float xj) { return A::density(P, xj); }, add_density, d);
     if (cross) {  // only state-0 high-res particles can contribute (lambda_LH)
         grid_coord_s<1>(P, p.x, p.y, -P.r, csx, csy);
         grid_coord_s<1>(P, p.x, p.y, P.r, cex, cey);
@@ -305,7 +362,7 @@ __device__ __forceinline__ void density_low_one(const Params& P, const StepView&
 
 template <bool B, class G, class A>
 __global__ void __launch_bounds__(256) k_density_low(Params P0, StepView V) {
-    __shared__ int16_t s_nbr[G::kWarp ? 1 : kMaxNbr * kNbrCols];
+    __shared__ int16_t s_nbr[G::kWarp ? 1 : kNbrRows * kNbrCols];
     int16_t* const nbr_col = s_nbr + (G::kWarp ? 0 : threadIdx.x);
     const bool cross = V.cnt->h_state0 != 0;
     for_each_particle<G>(V.cnt->cur[0], [&](int i) {

@@ -351,17 +351,19 @@ __global__ void __launch_bounds__(kReorderThreads) k_grid_reorder(int* n_ptr, in
     }
 }
 
-size_t grid_bufs_bytes(int cap, int ncells, bool own_off) {
+size_t grid_bufs_bytes(int cap, int ncells, bool own_off, bool own_sort) {
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
     int ntiles = (ncells + kScanTile - 1) / kScanTile;
     if (ntiles < 1) ntiles = 1;
     const size_t big_cap = static_cast<size_t>(cap) / (kBigCell + 1) + 1;
     return al(sizeof(unsigned) * (size_t)ncells) + (own_off ? al(sizeof(int) * ((size_t)ncells + 1)) : 0) +
-           al(sizeof(int) * (size_t)cap) * 3 + al(sizeof(int2) * (size_t)cap) + al(sizeof(unsigned) * (size_t)ntiles) +
+           al(sizeof(int) * (size_t)cap) * 2 +
+           (own_sort ? al(sizeof(int) * (size_t)cap) + al(sizeof(int2) * (size_t)cap) : 0) +
+           al(sizeof(unsigned) * (size_t)ntiles) +
            al(sizeof(int) * big_cap) + 256;
 }
 
-GridBufs grid_bufs_carve(void* base, int cap, int ncells, bool own_off) {
+GridBufs grid_bufs_carve(void* base, int cap, int ncells, bool own_off, bool own_sort) {
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
     char* p = static_cast<char*>(base);
     GridBufs g;
@@ -379,10 +381,14 @@ GridBufs grid_bufs_carve(void* base, int cap, int ncells, bool own_off) {
     p += al(sizeof(int) * (size_t)cap);
     g.rank = reinterpret_cast<int*>(p);
     p += al(sizeof(int) * (size_t)cap);
-    g.sortbuf = reinterpret_cast<int*>(p);
-    p += al(sizeof(int) * (size_t)cap);
-    g.perm = reinterpret_cast<int2*>(p);
-    p += al(sizeof(int2) * (size_t)cap);
+    g.sortbuf = nullptr;
+    g.perm = nullptr;
+    if (own_sort) {
+        g.sortbuf = reinterpret_cast<int*>(p);
+        p += al(sizeof(int) * (size_t)cap);
+        g.perm = reinterpret_cast<int2*>(p);
+        p += al(sizeof(int2) * (size_t)cap);
+    }
     g.tile_sum = reinterpret_cast<unsigned*>(p);
     p += al(sizeof(unsigned) * (size_t)g.ntiles);
     g.big_cap = cap / (kBigCell + 1) + 1;
@@ -393,6 +399,11 @@ GridBufs grid_bufs_carve(void* base, int cap, int ncells, bool own_off) {
     g.nbig = g.total + 1;
     g.nbig_snap = g.total + 2;
     return g;
+}
+
+void grid_lend_sort(GridBufs& g, void* mem, int cap) {
+    g.perm = static_cast<int2*>(mem);
+    g.sortbuf = reinterpret_cast<int*>(g.perm + cap);
 }
 
 cudaError_t grid_keys_enqueue(const float2* pos, const int* n_ptr, int cap, float ox, float oy, float cell, int dimx,

@@ -123,10 +123,14 @@ __device__ __forceinline__ void grid_key(unsigned* __restrict__ count, int* __re
     if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&tile_sum[t], static_cast<unsigned>(__popc(peers)));
 }
 
-// Device bytes of a grid's buffers for `cap` entries and `ncells` cells; own_off =
+// Device bytes of a grid's buffers for `cap` entries and `ncells` cells.  own_off =
 // false leaves out the offset table (the caller then sets g.off to its own).
-size_t grid_bufs_bytes(int cap, int ncells, bool own_off = true);
-GridBufs grid_bufs_carve(void* base, int cap, int ncells, bool own_off = true);
+// own_sort = false leaves out perm and sortbuf, which only live within a build: the
+// caller lends the build grid_sort_bytes(cap) that are dead then (grid_lend_sort).
+size_t grid_bufs_bytes(int cap, int ncells, bool own_off = true, bool own_sort = true);
+GridBufs grid_bufs_carve(void* base, int cap, int ncells, bool own_off = true, bool own_sort = true);
+constexpr size_t grid_sort_bytes(size_t cap) { return cap * (sizeof(int2) + sizeof(int)); }
+void grid_lend_sort(GridBufs& g, void* mem, int cap);
 
 int particle_blocks(int cap, int threads);
 int sm_count();

@@ -213,7 +213,6 @@ void plan_pool(tss_solver* s, const tss_pool_config& c, Arena& A, PoolPlan& pp) 
         A.add(&b.dens, cap);
         A.add(&b.pres, cap);
         A.add(&b.q, cap);
-        A.add(&b.tr, cap);
         A.add(&b.nbr, static_cast<size_t>(kMaxNbr) * (cap > 0 ? cap : 1));
         A.add(&b.nnbr, cap);
         b.cap = cap > 0 ? cap : 1;
@@ -222,11 +221,13 @@ void plan_pool(tss_solver* s, const tss_pool_config& c, Arena& A, PoolPlan& pp) 
     };
     scale(s->L, Ls, s->slotsL);
     scale(s->H, Hc > 0 ? Hc : 1, s->slotsH);
+    A.add(&s->L.tr, Ls);
+    A.add(&s->H.tr, 1);
     A.add(&s->L.cflag, CLc);
     A.add(&s->H.cflag, 1);
     A.add(&s->wnear, CLc);
-    A.add(&pp.gL, grid_bufs_bytes(Ls, CLc));
-    A.add(&pp.gH, grid_bufs_bytes(Hc > 0 ? Hc : 1, CHc));
+    A.add(&pp.gL, grid_bufs_bytes(Ls, CLc, true, false));
+    A.add(&pp.gH, grid_bufs_bytes(Hc > 0 ? Hc : 1, CHc, true, false));
     A.add(&pp.gW, grid_bufs_bytes(Wc > 0 ? Wc : 1, CLc));
     A.add(&s->wpos, Wc);
     A.add(&s->wraw, Wc);
@@ -276,8 +277,9 @@ tss_status create_pool(const tss_pool_config& c, bool reserve_high, tss_solver**
     }
     s->arena_bytes = A.total();
     A.carve(s->arena);
-    s->L.g = grid_bufs_carve(pp.gL, s->nL, s->CL);
-    s->H.g = grid_bufs_carve(pp.gH, s->capH > 0 ? s->capH : 1, s->CH);
+    s->L.g = grid_bufs_carve(pp.gL, s->nL, s->CL, true, false);
+    s->H.g = grid_bufs_carve(pp.gH, s->capH > 0 ? s->capH : 1, s->CH, true, false);
+    s->lend_lists();
     s->gW = grid_bufs_carve(pp.gW, s->capW > 0 ? s->capW : 1, s->CL);
     s->L.g.used = s->usedL;
     s->H.g.used = s->usedH;

@@ -509,7 +509,6 @@ tss_status create_solver(const SceneIn& sc, int cap_high, tss_solver** out) {
         A.add(&b.dens, cap);
         A.add(&b.pres, cap);
         A.add(&b.q, cap);
-        A.add(&b.tr, cap);
         A.add(&b.nbr, static_cast<size_t>(kMaxNbr) * (cap > 0 ? cap : 1));
         A.add(&b.nnbr, cap);
         b.cap = cap > 0 ? cap : 1;
@@ -518,14 +517,16 @@ tss_status create_solver(const SceneIn& sc, int cap_high, tss_solver** out) {
     };
     scale(s->L, n_low, s->slotsL);
     scale(s->H, cap_high, s->slotsH);
+    A.add(&s->L.tr, n_low);
+    A.add(&s->H.tr, 1);
     A.add(&s->L.cflag, s->CL);
     A.add(&s->H.cflag, 1);
     A.add(&s->wnear, s->CL);
     char* gL = nullptr;
     char* gH = nullptr;
     char* gW = nullptr;
-    A.add(&gL, grid_bufs_bytes(n_low > 0 ? n_low : 1, s->CL));
-    A.add(&gH, grid_bufs_bytes(cap_high > 0 ? cap_high : 1, s->CH));
+    A.add(&gL, grid_bufs_bytes(n_low > 0 ? n_low : 1, s->CL, true, false));
+    A.add(&gH, grid_bufs_bytes(cap_high > 0 ? cap_high : 1, s->CH, true, false));
     A.add(&gW, grid_bufs_bytes(n_wall > 0 ? n_wall : 1, s->CL));
     float2* wraw = nullptr;
     int32_t* wid = nullptr;
@@ -549,8 +550,9 @@ tss_status create_solver(const SceneIn& sc, int cap_high, tss_solver** out) {
     }
     s->arena_bytes = A.total();
     A.carve(s->arena);
-    s->L.g = grid_bufs_carve(gL, n_low > 0 ? n_low : 1, s->CL);
-    s->H.g = grid_bufs_carve(gH, cap_high > 0 ? cap_high : 1, s->CH);
+    s->L.g = grid_bufs_carve(gL, n_low > 0 ? n_low : 1, s->CL, true, false);
+    s->H.g = grid_bufs_carve(gH, cap_high > 0 ? cap_high : 1, s->CH, true, false);
+    s->lend_lists();
     GridBufs gw = grid_bufs_carve(gW, n_wall > 0 ? n_wall : 1, s->CL);
     s->woff = gw.off;
     // the low-res gathers take one block per 256 particles (their count is fixed):

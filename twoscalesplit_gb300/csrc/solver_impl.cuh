@@ -33,7 +33,9 @@ struct ScaleBufs {
     float *dens, *pres, *q, *ndens, *npres;
     float* tr;  // low scale: a split parent's tether radius this step (sorted order)
     uint8_t* cflag;  // low scale: per cell, the step stamp of a cell with an unsplit entry (see ScaleView)
-    int16_t* nbr;  // neighbour lists, kMaxNbr x cap (see ScaleView)
+    // neighbour lists, kMaxNbr x cap (see ScaleView); dead from the force pass to the
+    // next density pass, where the grid build keeps its permutation in them
+    int16_t* nbr;
     uint8_t* nnbr;
     int cap;       // entries of the sorted arrays
     GridBufs g;
@@ -228,6 +230,11 @@ struct tss_solver {
         return e == cudaErrorMemoryAllocation ? TSS_OOM : TSS_CUDA_ERROR;
     }
 
+    // the grid builds' permutations go where the neighbour lists are
+    void lend_lists() {
+        static_assert(tss::grid_sort_bytes(1) <= sizeof(int16_t) * tss::kMaxNbr, "a build's permutation fits the lists");
+        for (tss::ScaleBufs* b : {&L, &H}) tss::grid_lend_sort(b->g, b->nbr, b->cap);
+    }
     tss::StepView view() const;
     tss::ReorderArgs reorder_args(tss::ScaleBufs& b, bool high);
     cudaError_t mark(int k, cudaStream_t s);

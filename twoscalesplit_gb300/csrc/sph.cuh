@@ -64,7 +64,13 @@ struct StepView {
     const uint16_t* scH;
 };
 
-constexpr int kMaxNbr = 20;
+// The longest list.  A split parent's four children end up close together, so high-res
+// lists are 3 + 4 per neighbouring clump long: on a dam break of 1.0M high-res
+// particles 0.27 % of them have more than 20 neighbours, but 8 % of the warps hold one
+// and walk again (high-res density and force 93 and 151 us), and 0.005 % more than 24
+// (82 and 138 us; 28: 78 and 133).  24 is what fits without the handle's memory
+// growing: a grid build borrows the lists for its permutation (12 bytes an entry).
+constexpr int kMaxNbr = 24;
 constexpr uint8_t kNbrOverflow = 255;
 
 constexpr int kSplitThreads = 256;
