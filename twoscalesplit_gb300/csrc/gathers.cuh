@@ -68,7 +68,12 @@ using namespace gather_detail;
 // accept different candidates of the ~34 in their windows, so a walk that evaluates
 // a pair as soon as its test passes runs the pair arithmetic for nearly every
 // candidate with a third of the lanes active; here it runs once per list entry with
-// almost all of them (the lists are 10-14 long).
+// almost all of them (the lists are 10-14 long).  A dam break of 1.0M low-res and
+// 1.0M high-res particles, exact / tolerance arithmetic, against a walk that
+// evaluated at once: low-res density 96 -> 61 / 73 -> 51 us, high-res density 117 ->
+// 86 / 92 -> 67 us (with the longer lists, kMaxNbr); a 5,000-particle scene 16 -> 13
+// and 18 -> 12 us.  Warp instructions of the exact low-res density 94 -> 53 M, active
+// lanes 17 -> 26 of 32; issue still bounds it (79 % of cycles), DRAM a few percent.
 constexpr int kNbrCols = 256;          // the gathers' largest block
 constexpr int kNbrRows = kMaxNbr + 5;  // the particle itself, and one trip of four past a full list
 
