@@ -78,3 +78,16 @@ def test_rows_past_a_16_bit_offset():
     p = scenes.particle_box(0.5 * dx, 0.5 * dx, dx, nx, ny) + rng.uniform(-0.05 * dx, 0.05 * dx, size=(nx * ny, 2))
     sc = _scene(p, 2 * dx, (1.0, 8 * dx))
     _check(sc)
+
+
+@pytest.mark.parametrize("low_states,high_states", [([0, 1], [1]), ([0, 1, 2], [1]), ([0, 1, 2, 3], [0, 1, 2, 3])])
+def test_masks_of_every_state(low_states, high_states):
+    # the force passes read a neighbour's state only when a mask can reject it
+    rng = np.random.default_rng(8)
+    r, n = 0.02, 900
+    p = scenes.particle_box(0.1, 0.1, 0.5 * r, 30, 30) + rng.uniform(-0.1 * r, 0.1 * r, size=(n, 2))
+    sc = _scene(p, r, (0.6, 0.6))
+    hp = scenes.particle_box(0.15, 0.15, 0.25 * r, 40, 40) + rng.uniform(-0.05 * r, 0.05 * r, size=(1600, 2))
+    high = {"id": rng.permutation(3600)[:1600].astype(np.int32), "pos": hp.astype(np.float32),
+            "vel": rng.standard_normal((1600, 2)).astype(np.float32), "state": rng.choice(high_states, 1600).astype(np.uint8)}
+    _check(sc, high, rng.choice(low_states, n).astype(np.uint8))

@@ -33,6 +33,7 @@ namespace gather_detail {
 __device__ __forceinline__ int nthreads() { return gridDim.x * blockDim.x; }
 __device__ __forceinline__ int tid() { return blockIdx.x * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ float2 sub(float2 a, float2 b) { return sub2(a, b); }
+__device__ __forceinline__ float2 vel_of(float4 vq) { return make_float2(vq.x, vq.y); }
 __device__ __forceinline__ void add_density(float& d, float t) { d += t; }
 
 // The particles of a gather, one per thread (G = PerThread) or one per warp
@@ -148,45 +149,45 @@ __device__ __forceinline__ void nbr_density(const Params& P, const ScaleView& S,
 
 // A same-scale neighbour's state as the force pass reads it.
 struct NbrState {
-    float2 pos, vel;
-    float q, dens;
-    unsigned st;
+    int k;
+    float2 pos;
+    float4 vq;
 };
-__device__ __forceinline__ NbrState fetch_nbr(const ScaleView& S, int k) {
-    return NbrState{S.pos[k], S.vel[k], S.q[k], S.dens[k], S.st[k]};
-}
-
-// Entries of a neighbour list taken per trip of the force pass's list walk (1 or 2).
-constexpr int kListPairsPerTrip = 2;
+__device__ __forceinline__ NbrState fetch_nbr(const ScaleView& S, int k) { return NbrState{k, S.pos[k], S.vq[k]}; }
 
 // The force pass's same-scale pairs: from the list when there is one (test and
 // term take the neighbour's NbrState), else `walk`.  Two entries per trip: both
-// neighbours' state is loaded before either pair is evaluated, in list order, so
-// that a thread has two neighbours' loads in flight (the force kernels wait mostly
-// on these loads).  On a developed 1M-particle dam break that took k_force_high
-// from 0.149 to 0.133 ms (exact) and 0.110 to 0.094 ms (tolerance arithmetic)
-// against one per trip; four per trip was 3-8 % slower than two, with or without
-// one block per SM fewer for the registers.
+// neighbours' state is loaded before either pair is evaluated, in list order, and the
+// next trip's entries before them too, so that no trip waits for its entries and then
+// for its neighbours (the force kernels wait mostly on these loads).  An absent second
+// entry is taken as offset 0, the particle itself, which every force test rejects.
+// On a dam break of 1.0M + 1.0M particles, with a neighbour's velocity, p/rho^2 and
+// rho in one vector instead of three arrays (ScaleView::vq), the low-res force took
+// 97 -> 91 us (exact) and 68 -> 64 us (tolerance arithmetic), the high-res force 138 ->
+// 130 and 91 -> 86 us; one entry per trip instead of two costs 13-18 % of the high-res
+// force, four per trip 3-8 % (registers).  Two entries to a 32-bit word took 2 us off
+// the low-res force and put 3-5 us on each density.
 template <class G, class T, class Test, class Term, class Add, class Walk>
 __device__ __forceinline__ void list_or_walk(const ScaleView& S, int i, Test&& test, Term&& term, Add&& add,
                                              T& sum, Walk&& walk) {
     if constexpr (!G::kWarp) {
         const int nc = S.nbr ? S.nnbr[i] : kNbrOverflow;
         if (nc != kNbrOverflow) {
-            const long long stride = S.nbr_stride;
             const int16_t* src = S.nbr + i;
-            int c = 0;
-            if constexpr (kListPairsPerTrip == 2) {
-                for (; c + 1 < nc; c += 2, src += 2 * stride) {
-                    const int k0 = i + src[0], k1 = i + src[stride];
-                    const NbrState n0 = fetch_nbr(S, k0), n1 = fetch_nbr(S, k1);
-                    if (test(n0)) add(sum, term(n0));
-                    if (test(n1)) add(sum, term(n1));
-                }
-            }
-            for (; c < nc; ++c, src += stride) {
-                const NbrState n0 = fetch_nbr(S, i + *src);
+            int d0 = 0, d1 = 0;
+            const auto next = [&](int c) {
+                if (c < nc) d0 = *src;
+                src += S.nbr_stride;
+                d1 = 0;
+                if (c + 1 < nc) d1 = *src;
+                src += S.nbr_stride;
+            };
+            next(0);
+            for (int c = 0; c < nc; c += 2) {
+                const NbrState n0 = fetch_nbr(S, i + d0), n1 = fetch_nbr(S, i + d1);
+                next(c + 2);
                 if (test(n0)) add(sum, term(n0));
+                if (test(n1)) add(sum, term(n1));
             }
             return;
         }
@@ -294,7 +295,7 @@ __device__ __forceinline__ void density_high_one(const Params& P, const StepView
     if (G::leader()) {
         H.dens[i] = d;
         H.pres[i] = pr;
-        H.q[i] = pr / (d * d);
+        *reinterpret_cast<float2*>(&H.vq[i].z) = make_float2(pr / (d * d), d);
         if (!isfinite(d) || !isfinite(pr)) atomicOr(&V.cnt->err, kErrNumeric);
     }
 }
@@ -360,7 +361,7 @@ __device__ __forceinline__ void density_low_one(const Params& P, const StepView&
     if (G::leader()) {
         L.dens[i] = rho;
         L.pres[i] = pr;
-        L.q[i] = pr / (rho * rho);
+        *reinterpret_cast<float2*>(&L.vq[i].z) = make_float2(pr / (rho * rho), rho);
         if (!isfinite(rho) || !isfinite(pr)) atomicOr(&V.cnt->err, kErrNumeric);
     }
 }
@@ -425,12 +426,13 @@ __device__ __forceinline__ float2 wall_sum(const Params& P, const StepView& V, f
 // also gives the entry's key for the next step's grid.  Returns the split flag.
 // ---------------------------------------------------------------------------
 template <class A, class G>
-__device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V, int i, bool cross) {
+__device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V, int i, bool cross, bool deleted) {
     const ScaleView& H = V.H;
     const ScaleView& L = V.L;
-    float2 p = L.pos[i], v = L.vel[i];
+    const float4 own = L.vq[i];
+    float2 p = L.pos[i], v = vel_of(own);
     const unsigned s = L.st[i];
-    const float dens = L.dens[i], qi = L.q[i];
+    const float qi = own.z, dens = own.w;
     PairTerms fl{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};  // (acc, accT)
     float2 pij = make_float2(0.f, 0.f);
     float x = 0.0f;
@@ -444,15 +446,16 @@ __device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V
             return x != 0.0f && x <= P.Tlt_r && notDeleted(L.st[k]);
         };
         const auto term = [&](int j) {
-            return A::template pair<kHLow>(P, pij, x, sub(v, L.vel[j]), qi, L.q[j], dens, L.dens[j]);
+            const float4 o = L.vq[j];
+            return A::template pair<kHLow>(P, pij, x, sub(v, vel_of(o)), qi, o.z, dens, o.w);
         };
         const auto test_n = [&](const NbrState& n) {
             pij = sub(p, n.pos);
             x = sq(pij);
-            return x != 0.0f && x <= P.Tlt_r && notDeleted(n.st);
+            return x != 0.0f && x <= P.Tlt_r && (!deleted || notDeleted(L.st[n.k]));
         };
         const auto term_n = [&](const NbrState& n) {
-            return A::template pair<kHLow>(P, pij, x, sub(v, n.vel), qi, n.q, dens, n.dens);
+            return A::template pair<kHLow>(P, pij, x, sub(v, vel_of(n.vq)), qi, n.vq.z, dens, n.vq.w);
         };
         list_or_walk<G>(L, i, test_n, term_n, add_terms, fl,
                         [&] { G::window(L.off + P.cbL, P.dimL[0], csx, cex, csy, cey, test, term, add_terms, fl); });
@@ -471,7 +474,8 @@ __device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V
                 return x != 0.0f && x <= P.Tlt_r;
             },
             [&](int j) {
-                return A::template pair<kHCross>(P, pij, x, sub(v, H.vel[j]), qi, H.q[j], dens, H.dens[j]);
+                const float4 o = H.vq[j];
+                return A::template pair<kHCross>(P, pij, x, sub(v, vel_of(o)), qi, o.z, dens, o.w);
             },
             add_terms, fh);
     }
@@ -550,13 +554,13 @@ __device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V
 template <bool B, class G, class A>
 __global__ void __launch_bounds__(256, (A::kFast && !B) ? 6 : 5) k_force_low(Params P0, StepView V) {
     const int n = V.cnt->cur[0];
-    const bool cross = V.cnt->h_state0 != 0;
+    const bool cross = V.cnt->h_state0 != 0, deleted = V.cnt->l_deleted != 0;
     const auto one = [&](int i) {
         if constexpr (B) {
             const Params& P = V.table[V.scL[i]];
-            return force_low_one<A, G>(P, V, i, cross);
+            return force_low_one<A, G>(P, V, i, cross, deleted);
         } else {
-            return force_low_one<A, G>(P0, V, i, cross);
+            return force_low_one<A, G>(P0, V, i, cross, deleted);
         }
     };
     if constexpr (G::kWarp) {
@@ -584,9 +588,10 @@ template <class A, class G>
 __device__ __forceinline__ void force_high_one(const Params& P, const StepView& V, int i) {
     const ScaleView& H = V.H;
     const ScaleView& L = V.L;
-    float2 p = H.pos[i], v = H.vel[i];
+    const float4 own = H.vq[i];
+    float2 p = H.pos[i], v = vel_of(own);
     const unsigned s = H.st[i];
-    const float dens = H.dens[i], qi = H.q[i];
+    const float qi = own.z, dens = own.w;
     PairTerms fh{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};  // (acc, accT)
     float2 pij = make_float2(0.f, 0.f);
     float x = 0.0f;
@@ -601,16 +606,16 @@ __device__ __forceinline__ void force_high_one(const Params& P, const StepView& 
             return x != 0.0f && x <= P.Tlt_rh;
         };
         const auto term = [&](int j) {
-            return A::template pair<kHHigh>(P, pij, x, sub(v, H.vel[j]), qi, H.q[j], dens, H.dens[j]);
+            const float4 o = H.vq[j];
+            return A::template pair<kHHigh>(P, pij, x, sub(v, vel_of(o)), qi, o.z, dens, o.w);
         };
         const auto test_n = [&](const NbrState& n) {
-            if (!lamHH(s, n.st)) return false;
             pij = sub(p, n.pos);
             x = sq(pij);
-            return x != 0.0f && x <= P.Tlt_rh;
+            return x != 0.0f && x <= P.Tlt_rh && ((s & 1u) || lamHH(s, H.st[n.k]));
         };
         const auto term_n = [&](const NbrState& n) {
-            return A::template pair<kHHigh>(P, pij, x, sub(v, n.vel), qi, n.q, dens, n.dens);
+            return A::template pair<kHHigh>(P, pij, x, sub(v, vel_of(n.vq)), qi, n.vq.z, dens, n.vq.w);
         };
         list_or_walk<G>(H, i, test_n, term_n, add_terms, fh,
                         [&] { G::window(H.off + P.cbH, P.dimH[0], csx, cex, csy, cey, test, term, add_terms, fh); });
@@ -640,7 +645,8 @@ __device__ __forceinline__ void force_high_one(const Params& P, const StepView& 
             return x != 0.0f && x <= P.Tlt_r;
         },
         [&](int j) {
-            return A::template pair<kHCross>(P, pij, x, sub(v, L.vel[j]), qi, L.q[j], dens, L.dens[j]);
+            const float4 o = L.vq[j];
+            return A::template pair<kHCross>(P, pij, x, sub(v, vel_of(o)), qi, o.z, dens, o.w);
         },
         add_terms, fl);
     const float2 accB = wall_sum<A, G, 1>(P, V, p, csx, cex, csy, cey, P.Tle_rh, P.cBH);

@@ -178,11 +178,12 @@ namespace {
 // Gathers list entry src's state into sorted position dst.
 __device__ __forceinline__ void reorder_move(const ReorderArgs& a, int src, int dst, int id, unsigned* err) {
     if (a.dst_pos) a.dst_pos[dst] = a.src_pos[src];
-    if (a.src_vel) a.dst_vel[dst] = a.src_vel[src];
+    if (a.src_vel) *reinterpret_cast<float2*>(&a.dst_vq[dst]) = a.src_vel[src];
     if (a.src_st) {
         uint8_t st = a.src_st[src];
         a.dst_st[dst] = st;
         if (a.h_state0 && (st & 1u) == 0u) *a.h_state0 = 1;
+        if (a.deleted && st >= 2u) *a.deleted = 1;
     }
     if (a.dst_id) a.dst_id[dst] = id;
     if (a.src_dens) {

@@ -71,7 +71,7 @@ struct ReorderArgs {
     const float* src_dens;     // may be null (carried only for the relaxation)
     const float* src_pres;
     float2* dst_pos;
-    float2* dst_vel;
+    float4* dst_vq;            // the velocity goes to .xy
     uint8_t* dst_st;
     int32_t* dst_id;
     float* dst_dens;
@@ -86,6 +86,7 @@ struct ReorderArgs {
     int page_shift;
     int id_shift;              // 0 for low-res ids, 2 for high-res (4 children per parent)
     int* h_state0;             // may be null: set to 1 if some entry has (state & 1) == 0
+    int* deleted;              // may be null: set to 1 if some entry has state >= 2
 };
 
 __global__ void k_grid_keys(const float2* __restrict__ pos, const int* __restrict__ n_ptr, float ox, float oy,

@@ -201,7 +201,7 @@ void plan_pool(tss_solver* s, const tss_pool_config& c, Arena& A, PoolPlan& pp) 
     s->S = c.max_scenes;
     auto scale = [&](ScaleBufs& b, int cap, int slots) {
         A.add(&b.pos, cap);
-        A.add(&b.vel, cap);
+        A.add(&b.vq, cap);
         A.add(&b.acc, cap);
         A.add(&b.npos, cap);
         A.add(&b.nvel, cap);
@@ -212,7 +212,6 @@ void plan_pool(tss_solver* s, const tss_pool_config& c, Arena& A, PoolPlan& pp) 
         A.add(&b.map, slots);
         A.add(&b.dens, cap);
         A.add(&b.pres, cap);
-        A.add(&b.q, cap);
         A.add(&b.nbr, static_cast<size_t>(kMaxNbr) * (cap > 0 ? cap : 1));
         A.add(&b.nnbr, cap);
         b.cap = cap > 0 ? cap : 1;

@@ -19,12 +19,11 @@ StepView tss_solver::view() const {
     auto sv = [](const ScaleBufs& b) {
         ScaleView s{};
         s.pos = b.pos;
-        s.vel = b.vel;
+        s.vq = b.vq;
         s.st = b.st;
         s.id = b.id;
         s.dens = b.dens;
         s.pres = b.pres;
-        s.q = b.q;
         s.tr = b.tr;
         s.cflag = b.cflag;
         s.nbr = b.nbr;
@@ -73,7 +72,7 @@ ReorderArgs tss_solver::reorder_args(ScaleBufs& b, bool high) {
     a.src_vel = b.nvel;
     a.src_st = b.nst;
     a.dst_pos = b.pos;
-    a.dst_vel = b.vel;
+    a.dst_vq = b.vq;
     a.dst_st = b.st;
     a.dst_id = b.id;
     a.slot_map = b.map;
@@ -85,6 +84,7 @@ ReorderArgs tss_solver::reorder_args(ScaleBufs& b, bool high) {
         a.dst_pres = b.pres;
     }
     if (high) a.h_state0 = &cnt->h_state0;
+    else a.deleted = &cnt->l_deleted;
     if (batched) {
         a.dst_sc = high ? scH : scL;
         a.page_scene = page_scene;
@@ -247,7 +247,7 @@ __global__ void k_fill_i32(int32_t* p, int64_t n, int v) {
 __global__ void k_set_counts(Counters* c, int nL, int nH) {
     c->cur[0] = c->next[0] = nL;
     c->cur[1] = c->next[1] = nH;
-    c->h_state0 = 0;
+    c->h_state0 = c->l_deleted = 0;
     c->n_drop = c->dropped = 0;
 }
 __global__ void k_set_fresh(Counters* c, int n) { c->n_fresh = n; }
@@ -497,7 +497,7 @@ tss_status create_solver(const SceneIn& sc, int cap_high, tss_solver** out) {
     Arena A;
     auto scale = [&](ScaleBufs& b, int cap, int slots) {
         A.add(&b.pos, cap);
-        A.add(&b.vel, cap);
+        A.add(&b.vq, cap);
         A.add(&b.acc, cap);
         A.add(&b.npos, cap);
         A.add(&b.nvel, cap);
@@ -508,7 +508,6 @@ tss_status create_solver(const SceneIn& sc, int cap_high, tss_solver** out) {
         A.add(&b.map, slots);
         A.add(&b.dens, cap);
         A.add(&b.pres, cap);
-        A.add(&b.q, cap);
         A.add(&b.nbr, static_cast<size_t>(kMaxNbr) * (cap > 0 ? cap : 1));
         A.add(&b.nnbr, cap);
         b.cap = cap > 0 ? cap : 1;

@@ -27,10 +27,11 @@
 namespace tss {
 
 struct ScaleBufs {
-    float2 *pos, *vel, *acc, *npos, *nvel;
+    float2 *pos, *acc, *npos, *nvel;
+    float4* vq;  // (velocity, p/rho^2, rho), see ScaleView
     uint8_t *st, *nst;
     int32_t *id, *nid, *map;
-    float *dens, *pres, *q, *ndens, *npres;
+    float *dens, *pres, *ndens, *npres;
     float* tr;  // low scale: a split parent's tether radius this step (sorted order)
     uint8_t* cflag;  // low scale: per cell, the step stamp of a cell with an unsplit entry (see ScaleView)
     // neighbour lists, kMaxNbr x cap (see ScaleView); dead from the force pass to the

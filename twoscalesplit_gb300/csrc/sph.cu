@@ -193,7 +193,7 @@ __device__ __forceinline__ void relax_force_one(const Params& P, const StepView&
     const int* offL = L.off + P.cbL;
     const int* woff = V.woff + P.cbL;
     const float2* wpos = V.wpos + P.wb;
-    float2 p = H.pos[i], v = H.vel[i];
+    float2 p = H.pos[i], v = vel_of(H.vq[i]);
     const float dens = H.dens[i], pre = H.pres[i];
     const float dens2 = dens * dens;
     float2 acc = make_float2(0.f, 0.f), accL = make_float2(0.f, 0.f), accB = make_float2(0.f, 0.f);
@@ -276,7 +276,7 @@ __global__ void k_relax_apply(Params P0, StepView V) {
         const int i = fresh_child(P0, V, f);
         if (i < 0) continue;
         const_cast<float2*>(V.H.pos)[i] = V.relax_pos[f];
-        const_cast<float2*>(V.H.vel)[i] = V.relax_vel[f];
+        *reinterpret_cast<float2*>(&V.H.vq[i]) = V.relax_vel[f];
     }
 }
 
@@ -287,7 +287,7 @@ __global__ void k_step_finish(Counters* c) {
         c->cur[0] = c->next[0];
         c->cur[1] = c->next[1];
         c->n_fresh = c->n_split;
-        c->h_state0 = 0;
+        c->h_state0 = c->l_deleted = 0;
         c->steps += 1;
         c->dropped = c->n_drop;
         c->total_split += c->n_split;

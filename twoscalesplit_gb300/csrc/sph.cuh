@@ -10,12 +10,15 @@ namespace tss {
 // existing particles, with newly created high-res children appended.
 struct ScaleView {
     const float2* pos;
-    const float2* vel;
+    // velocity (.xy, written by the grid build), p / rho^2 (.z) and rho (.w, both written
+    // by the density pass): with pos, what a force pair needs of a neighbour, in one
+    // 16-byte load.  As four arrays (and a state byte for every pair) the force kernels
+    // waited on five loads a neighbour instead of two.
+    float4* vq;
     const uint8_t* st;
     const int32_t* id;
     float* dens;
     float* pres;
-    float* q;        // p / rho^2
     float* tr;       // low scale: each split parent's tether radius, written by the low-res force
     // low scale, one byte per cell: the low-res force sets a cell to the step counter
     // (mod 256) when the cell holds an entry in state 0 after the split marks.  Any
