@@ -433,9 +433,10 @@ typedef struct tss_launch {
     int persistent[TSS_NUM_GATHERS];  /* 0: blocks cover the list's capacity (at most 4096 threads
                                          per SM, grid-striding beyond); 1: one wave of resident
                                          blocks (SMs x blocks per SM), each striding over the list */
-    int per_warp[TSS_NUM_GATHERS];    /* 0: one particle per thread (32 per warp); 1: one particle
-                                         per warp, its candidates spread over the lanes (for
-                                         scenes too small to fill the GPU)                         */
+    int per_warp[TSS_NUM_GATHERS];    /* 0: one particle per thread (32 per warp), or per group of 4
+                                         or 8 lanes while the list is too short to fill the GPU so;
+                                         1: one particle per warp, its candidates spread over the
+                                         lanes                                                     */
 } tss_launch;
 tss_status tss_solver_get_launch(tss_solver* s, tss_launch* out);
 /* Replaces the launch shape (the step graphs are captured again at the next step). */

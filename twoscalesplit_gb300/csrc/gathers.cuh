@@ -36,16 +36,40 @@ __device__ __forceinline__ float2 sub(float2 a, float2 b) { return sub2(a, b); }
 __device__ __forceinline__ float2 vel_of(float4 vq) { return make_float2(vq.x, vq.y); }
 __device__ __forceinline__ void add_density(float& d, float t) { d += t; }
 
-// The particles of a gather, one per thread (G = PerThread) or one per warp
-// (G = PerWarp, every lane of the warp taking the same particle).
+// The particles of a gather, one per thread (G = PerThread) or one per group of lanes
+// (PerGroup, every lane of a group taking the same particle).  f(i, valid): the
+// groups of a warp come together, those past the end with the last particle and
+// valid = false.
 template <class G, class F>
 __device__ __forceinline__ void for_each_particle(int n, F&& f) {
-    if constexpr (G::kWarp) {
-        const int nw = nthreads() >> 5;
-        for (int i = tid() >> 5; i < n; i += nw) f(i);
+    if constexpr (G::kLanes > 1) {
+        constexpr int per = 32 / G::kLanes;  // particles per warp
+        for (int base = (tid() >> 5) * per; base < n; base += (nthreads() >> 5) * per) {
+            const int i = base + (static_cast<int>(threadIdx.x) & 31) / G::kLanes;
+            f(min(i, n - 1), i < n);
+        }
     } else {
-        for (int i = tid(); i < n; i += nthreads()) f(i);
+        for (int i = tid(); i < n; i += nthreads()) f(i, true);
     }
+}
+
+// f(form, n) with the form that takes n particles: the launch's own, except that one
+// particle per thread becomes one per group of lanes for a short list (sph.cuh).
+template <class G, bool Force, class F>
+__device__ __forceinline__ void by_size(int n, F&& f) {
+    if constexpr (G::kLanes == 1) {
+        if (n <= (Force ? kForce8Max : kDensity8Max)) {
+            f(PerGroup<8>{}, n);
+            return;
+        }
+        if constexpr (Force) {
+            if (n <= kForce4Max) {
+                f(PerGroup<4>{}, n);
+                return;
+            }
+        }
+    }
+    f(G{}, n);
 }
 }  // namespace gather_detail
 using namespace gather_detail;
@@ -167,13 +191,36 @@ __device__ __forceinline__ NbrState fetch_nbr(const ScaleView& S, int k) { retur
 // 130 and 91 -> 86 us; one entry per trip instead of two costs 13-18 % of the high-res
 // force, four per trip 3-8 % (registers).  Two entries to a 32-bit word took 2 us off
 // the low-res force and put 3-5 us on each density.
+//
+// A group of lanes takes an entry per lane, up to three rounds of entries loaded
+// first.
 template <class G, class T, class Test, class Term, class Add, class Walk>
-__device__ __forceinline__ void list_or_walk(const ScaleView& S, int i, Test&& test, Term&& term, Add&& add,
+__device__ __forceinline__ void list_or_walk(bool on, const ScaleView& S, int i, Test&& test, Term&& term, Add&& add,
                                              T& sum, Walk&& walk) {
-    if constexpr (!G::kWarp) {
-        const int nc = S.nbr ? S.nnbr[i] : kNbrOverflow;
-        if (nc != kNbrOverflow) {
-            const int16_t* src = S.nbr + i;
+    const int nc = S.nnbr[i];
+    const bool listed = nc != kNbrOverflow;
+    const int16_t* src = S.nbr + i;
+    if constexpr (G::kLanes > 1) {
+        constexpr int kRounds = (kMaxNbr + G::kLanes - 1) / G::kLanes;
+        const int m = on && listed ? nc : 0;
+        int dj[kRounds];
+#pragma unroll
+        for (int r = 0; r < kRounds; ++r) {
+            const int c = r * G::kLanes + G::lane();
+            dj[r] = c < m ? src[c * S.nbr_stride] : 0;
+        }
+#pragma unroll
+        for (int r = 0; r < kRounds; ++r) {
+            if (!G::any(r * G::kLanes < m)) break;
+            const NbrState n0 = fetch_nbr(S, i + dj[r]);  // an absent entry is the particle itself: rejected
+            T t{};
+            const bool ok = r * G::kLanes + G::lane() < m && test(n0);
+            if (ok) t = term(n0);
+            G::add_lanes(G::ballot(ok), t, add, sum);
+        }
+        if (G::any(on && !listed)) walk(on && !listed);
+    } else {
+        if (listed) {
             int d0 = 0, d1 = 0;
             const auto next = [&](int c) {
                 if (c < nc) d0 = *src;
@@ -189,17 +236,66 @@ __device__ __forceinline__ void list_or_walk(const ScaleView& S, int i, Test&& t
                 if (test(n0)) add(sum, term(n0));
                 if (test(n1)) add(sum, term(n1));
             }
-            return;
+        } else {
+            walk(true);
         }
     }
-    walk();
+}
+
+// A particle's same-scale density sum over its window (candidates k with key(k) <= T),
+// which also records its neighbour list: in the two phases above, or, by a group of
+// lanes, W candidates at a time.
+template <class A, class G, class Key>
+__device__ __forceinline__ void same_scale_density(bool on, const Params& P, const ScaleView& S, const int* off,
+                                                   int dimx, int csx, int cex, int csy, int cey, int i, float2 p,
+                                                   float T, int16_t* nbr_col, float& sum, Key&& key) {
+    if constexpr (G::kLanes > 1) {
+        int n = 0;
+        bool fit = true;
+        for (int cy = csy; G::any(on && cy <= cey); ++cy) {
+            const int row = cy * dimx;
+            const bool in = on && cy <= cey;
+            const int a = in ? off[row + csx] : 0, b = in ? off[row + cex + 1] : 0;
+            if (in && (a - i < -32768 || b - i > 32768)) fit = false;
+            for (int base = a; G::any(base < b); base += G::kLanes) {
+                const int k = base + G::lane();
+                const float x = k < b ? key(k) : INFINITY;
+                const bool ok = x <= T;
+                const unsigned m = G::ballot(ok);
+                const int own = i - base;  // the particle itself is left out of the list
+                const unsigned listed = own >= 0 && own < G::kLanes ? m & ~(1u << own) : m;
+                if (ok && k != i) {
+                    const int c = n + __popc(listed & ((1u << G::lane()) - 1u));
+                    if (c < kMaxNbr && fit) S.nbr[c * S.nbr_stride + i] = static_cast<int16_t>(k - i);
+                }
+                n += __popc(listed);
+                G::add_lanes(m, ok ? A::density(P, x) : 0.0f, add_density, sum);
+            }
+        }
+        if (on && G::leader()) S.nnbr[i] = n <= kMaxNbr && fit ? static_cast<uint8_t>(n) : kNbrOverflow;
+    } else {
+        const int n = nbr_search(off, dimx, csx, cex, csy, cey, i, T, nbr_col, key);
+        if (n >= 0) {
+            nbr_density<A>(P, S, i, p, n, nbr_col, sum);
+        } else {
+            S.nnbr[i] = kNbrOverflow;
+            float x = 0.0f;
+            G::window(
+                true, off, dimx, csx, cex, csy, cey,
+                [&](int k) {
+                    x = key(k);
+                    return x <= T;
+                },
+                [&](int) { return A::density(P, x); }, add_density, sum);
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
 // High-res density + Tait, computeParticleDensityPressureHigh (WCSPHSolver.cu:1426-1516)
 // ---------------------------------------------------------------------------
 template <class A, class G>
-__device__ __forceinline__ void density_high_one(const Params& P, const StepView& V, int i, bool hstate0,
+__device__ __forceinline__ void density_high_one(const Params& P, const StepView& V, int i, bool valid, bool hstate0,
                                                  int16_t* nbr_col) {
     const ScaleView& H = V.H;
     const ScaleView& L = V.L;
@@ -213,22 +309,14 @@ __device__ __forceinline__ void density_high_one(const Params& P, const StepView
     int csx, csy, cex, cey;
     grid_coord_s<1>(P, p.x, p.y, -P.rh, csx, csy);
     grid_coord_s<1>(P, p.x, p.y, P.rh, cex, cey);
-    // a candidate the lambda mask rejects gets key +inf: no cutoff passes it
+    // a candidate the lambda mask rejects gets key +inf: no cutoff passes it (the mask
+    // passes every candidate of a state-1 particle)
     const auto masked = [&](int k) { return lamHH(s, H.st[k]) ? sq(sub(p, H.pos[k])) : INFINITY; };
-    int nn = -1;
-    if constexpr (!G::kWarp) {
-        if (s & 1u)  // the mask passes every candidate of a state-1 particle
-            nn = nbr_search(offH, P.dimH[0], csx, cex, csy, cey, i, P.Tle_rh, nbr_col,
-                            [&](int k) { return sq(sub(p, H.pos[k])); });
-        else
-            nn = nbr_search(offH, P.dimH[0], csx, cex, csy, cey, i, P.Tle_rh, nbr_col, masked);
-        if (nn >= 0) nbr_density<A>(P, H, i, p, nn, nbr_col, d);
-        else H.nnbr[i] = kNbrOverflow;
-    }
-    if (nn < 0)
-        G::window_keyed(
-            offH, P.dimH[0], csx, cex, csy, cey, masked, [&](float xk) { return xk <= P.Tle_rh; },
-            [&](int, float xj) { return A::density(P, xj); }, add_density, d);
+    const auto plain = [&](int k) { return sq(sub(p, H.pos[k])); };
+    if (!G::any((s & 1u) == 0u))
+        same_scale_density<A, G>(valid, P, H, offH, P.dimH[0], csx, cex, csy, cey, i, p, P.Tle_rh, nbr_col, d, plain);
+    else
+        same_scale_density<A, G>(valid, P, H, offH, P.dimH[0], csx, cex, csy, cey, i, p, P.Tle_rh, nbr_col, d, masked);
     grid_coord_s<0>(P, p.x, p.y, -P.r, csx, csy);
     grid_coord_s<0>(P, p.x, p.y, P.r, cex, cey);
     // With no high-res entry in state 0 in this step (hstate0 false), a state-1
@@ -237,7 +325,8 @@ __device__ __forceinline__ void density_high_one(const Params& P, const StepView
     // particle lies within r_h of (0,0): otherwise the walk adds nothing and is
     // skipped -- the same terms, none.
     const bool q1_live = hstate0 || (s & 1u) == 0u || sq(p) <= P.Tle_rh;
-    if (P.q1 && q1_live) {
+    const bool q1 = valid && P.q1 && q1_live;
+    if (G::any(q1)) {
         // The reference reads the HIGH sorted list at LOW-grid ranges of its own
         // scene; past the scene's n_high that list still holds its initial identity
         // (slot t at position t).  A row's range [a, b) of low-list positions t
@@ -248,9 +337,10 @@ __device__ __forceinline__ void density_high_one(const Params& P, const StepView
         const int nHs = offH[P.CHs] - baseH;
         const int tH = baseL + nHs;   // first position past the scene's high-res list
         const int dH = baseH - baseL;  // low-list position -> high-list entry
-        for (int cy = csy; cy <= cey; ++cy) {
+        for (int cy = csy; G::any(q1 && cy <= cey); ++cy) {
             const int row = cy * P.dimL[0];
-            const int a = offL[row + csx], b = offL[row + cex + 1];
+            const bool in = q1 && cy <= cey;
+            const int a = in ? offL[row + csx] : 0, b = in ? offL[row + cex + 1] : 0;
             const int m = min(b, max(a, tH));
             G::span(
                 a + dH, m + dH,
@@ -278,9 +368,10 @@ __device__ __forceinline__ void density_high_one(const Params& P, const StepView
                 },
                 term, add_density, d);
         }
-    } else if (!P.q1) {
+    }
+    if (G::any(valid && !P.q1)) {
         G::window(
-            offL, P.dimL[0], csx, cex, csy, cey,
+            valid && !P.q1, offL, P.dimL[0], csx, cex, csy, cey,
             [&](int k) {
                 if (!lamHL(s, L.st[k])) return false;
                 x = sq(sub(p, L.pos[k]));
@@ -292,7 +383,7 @@ __device__ __forceinline__ void density_high_one(const Params& P, const StepView
     dl *= P.mL;
     d += dl;
     const float pr = tait(d, P);
-    if (G::leader()) {
+    if (valid && G::leader()) {
         H.dens[i] = d;
         H.pres[i] = pr;
         *reinterpret_cast<float2*>(&H.vq[i].z) = make_float2(pr / (d * d), d);
@@ -301,17 +392,20 @@ __device__ __forceinline__ void density_high_one(const Params& P, const StepView
 }
 
 template <bool B, class G, class A>
-__global__ void __launch_bounds__(256) k_density_high(Params P0, StepView V) {
-    __shared__ int16_t s_nbr[G::kWarp ? 1 : kNbrRows * kNbrCols];
-    int16_t* const nbr_col = s_nbr + (G::kWarp ? 0 : threadIdx.x);
+__global__ void __launch_bounds__(256, B ? (A::kFast ? 6 : 5) : (A::kFast ? 8 : 6)) k_density_high(Params P0, StepView V) {
+    __shared__ int16_t s_nbr[G::kLanes > 1 ? 1 : kNbrRows * kNbrCols];
+    int16_t* const nbr_col = s_nbr + (G::kLanes > 1 ? 0 : threadIdx.x);
     const bool hstate0 = V.cnt->h_state0 != 0;
-    for_each_particle<G>(V.cnt->cur[1], [&](int i) {
-        if constexpr (B) {
-            const Params& P = V.table[V.scH[i]];
-            density_high_one<A, G>(P, V, i, hstate0, nbr_col);
-        } else {
-            density_high_one<A, G>(P0, V, i, hstate0, nbr_col);
-        }
+    by_size<G, false>(V.cnt->cur[1], [&](auto form, int n) {
+        using F = decltype(form);
+        for_each_particle<F>(n, [&](int i, bool valid) {
+            if constexpr (B) {
+                const Params& P = V.table[V.scH[i]];
+                density_high_one<A, F>(P, V, i, valid, hstate0, nbr_col);
+            } else {
+                density_high_one<A, F>(P0, V, i, valid, hstate0, nbr_col);
+            }
+        });
     });
 }
 
@@ -319,7 +413,7 @@ __global__ void __launch_bounds__(256) k_density_high(Params P0, StepView V) {
 // Low-res density + Tait, computeParticleDensityPressure (WCSPHSolver.cu:1342-1424)
 // ---------------------------------------------------------------------------
 template <class A, class G>
-__device__ __forceinline__ void density_low_one(const Params& P, const StepView& V, int i, bool cross,
+__device__ __forceinline__ void density_low_one(const Params& P, const StepView& V, int i, bool valid, bool cross,
                                                 int16_t* nbr_col) {
     const ScaleView& H = V.H;
     const ScaleView& L = V.L;
@@ -331,22 +425,13 @@ __device__ __forceinline__ void density_low_one(const Params& P, const StepView&
     int csx, csy, cex, cey;
     grid_coord_s<0>(P, p.x, p.y, -P.r, csx, csy);
     grid_coord_s<0>(P, p.x, p.y, P.r, cex, cey);
-    const auto key = [&](int k) { return sq(sub(p, L.pos[k])); };
-    int nn = -1;
-    if constexpr (!G::kWarp) {
-        nn = nbr_search(L.off + P.cbL, P.dimL[0], csx, cex, csy, cey, i, P.Tle_r, nbr_col, key);
-        if (nn >= 0) nbr_density<A>(P, L, i, p, nn, nbr_col, d);
-        else L.nnbr[i] = kNbrOverflow;
-    }
-    if (nn < 0)
-        G::window_keyed(
-            L.off + P.cbL, P.dimL[0], csx, cex, csy, cey, key, [&](float xk) { return xk <= P.Tle_r; },
-            [&](int, float xj) { return A::density(P, xj); }, add_density, d);
+    same_scale_density<A, G>(valid, P, L, L.off + P.cbL, P.dimL[0], csx, cex, csy, cey, i, p, P.Tle_r, nbr_col, d,
+                             [&](int k) { return sq(sub(p, L.pos[k])); });
     if (cross) {  // only state-0 high-res particles can contribute (lambda_LH)
         grid_coord_s<1>(P, p.x, p.y, -P.r, csx, csy);
         grid_coord_s<1>(P, p.x, p.y, P.r, cex, cey);
         G::window(
-            H.off + P.cbH, P.dimH[0], csx, cex, csy, cey,
+            valid, H.off + P.cbH, P.dimH[0], csx, cex, csy, cey,
             [&](int k) {
                 if (!lamLH(s, H.st[k])) return false;
                 x = sq(sub(p, H.pos[k]));
@@ -358,7 +443,7 @@ __device__ __forceinline__ void density_low_one(const Params& P, const StepView&
     dh *= P.mH;
     const float rho = d + dh;
     const float pr = tait(rho, P);
-    if (G::leader()) {
+    if (valid && G::leader()) {
         L.dens[i] = rho;
         L.pres[i] = pr;
         *reinterpret_cast<float2*>(&L.vq[i].z) = make_float2(pr / (rho * rho), rho);
@@ -367,17 +452,20 @@ __device__ __forceinline__ void density_low_one(const Params& P, const StepView&
 }
 
 template <bool B, class G, class A>
-__global__ void __launch_bounds__(256) k_density_low(Params P0, StepView V) {
-    __shared__ int16_t s_nbr[G::kWarp ? 1 : kNbrRows * kNbrCols];
-    int16_t* const nbr_col = s_nbr + (G::kWarp ? 0 : threadIdx.x);
+__global__ void __launch_bounds__(256, B ? 6 : 8) k_density_low(Params P0, StepView V) {
+    __shared__ int16_t s_nbr[G::kLanes > 1 ? 1 : kNbrRows * kNbrCols];
+    int16_t* const nbr_col = s_nbr + (G::kLanes > 1 ? 0 : threadIdx.x);
     const bool cross = V.cnt->h_state0 != 0;
-    for_each_particle<G>(V.cnt->cur[0], [&](int i) {
-        if constexpr (B) {
-            const Params& P = V.table[V.scL[i]];
-            density_low_one<A, G>(P, V, i, cross, nbr_col);
-        } else {
-            density_low_one<A, G>(P0, V, i, cross, nbr_col);
-        }
+    by_size<G, false>(V.cnt->cur[0], [&](auto form, int n) {
+        using F = decltype(form);
+        for_each_particle<F>(n, [&](int i, bool valid) {
+            if constexpr (B) {
+                const Params& P = V.table[V.scL[i]];
+                density_low_one<A, F>(P, V, i, valid, cross, nbr_col);
+            } else {
+                density_low_one<A, F>(P0, V, i, valid, cross, nbr_col);
+            }
+        });
     });
 }
 
@@ -386,35 +474,33 @@ __global__ void __launch_bounds__(256) k_density_low(Params P0, StepView V) {
 // sqrtf(x) > rad have q >= 2 and add exactly zero, so they are skipped.  S selects
 // the scale: 0 the low-res radius r, 1 the high-res radius rh.
 template <class A, class G, int S>
-__device__ __forceinline__ float2 wall_sum(const Params& P, const StepView& V, float2 p, int csx, int cex, int csy,
-                                           int cey, float Tle, float cB) {
+__device__ __forceinline__ float2 wall_sum(bool on, const Params& P, const StepView& V, float2 p, int csx, int cex,
+                                           int csy, int cey, float Tle, float cB) {
     float2 accB = make_float2(0.f, 0.f);
     // A window of at most four cells a side from (csx, csy) lies within two cells of
     // (mx, my); with no wall particle there the sum is empty.
     if (cex - csx <= 3 && cey - csy <= 3) {
         const int mx = min(csx + 1, P.dimL[0] - 1), my = min(csy + 1, P.dimL[1] - 1);
-        if (!V.wnear[P.cbL + my * P.dimL[0] + mx]) return accB;
+        on = on && V.wnear[P.cbL + my * P.dimL[0] + mx];
     }
+    if (!G::any(on)) return accB;
     const int* woff = V.woff + P.cbL;
     const float2* wpos = V.wpos + P.wb;
     float2 pik = make_float2(0.f, 0.f);
     float x = 0.0f;
-    for (int cy = csy; cy <= cey; ++cy) {
-        const int row = cy * P.dimL[0];
-        G::span(
-            woff[row + csx], woff[row + cex + 1],
-            [&](int k) {
-                pik = sub(p, wpos[k]);
-                x = sq(pik);
-                return !(x > Tle);  // NaN passes: the reference's 0 * NaN offset propagates it
-            },
-            [&](int) { return A::template wall<S>(P, pik, x, cB); },
-            [](float2& a, float2 t) {
-                a.x += t.x;
-                a.y += t.y;
-            },
-            accB);
-    }
+    G::window(
+        on, woff, P.dimL[0], csx, cex, csy, cey,
+        [&](int k) {
+            pik = sub(p, wpos[k]);
+            x = sq(pik);
+            return !(x > Tle);  // NaN passes: the reference's 0 * NaN offset propagates it
+        },
+        [&](int) { return A::template wall<S>(P, pik, x, cB); },
+        [](float2& a, float2 t) {
+            a.x += t.x;
+            a.y += t.y;
+        },
+        accB);
     return accB;
 }
 
@@ -426,7 +512,8 @@ __device__ __forceinline__ float2 wall_sum(const Params& P, const StepView& V, f
 // also gives the entry's key for the next step's grid.  Returns the split flag.
 // ---------------------------------------------------------------------------
 template <class A, class G>
-__device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V, int i, bool cross, bool deleted) {
+__device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V, int i, bool valid, bool cross,
+                                              bool deleted) {
     const ScaleView& H = V.H;
     const ScaleView& L = V.L;
     const float4 own = L.vq[i];
@@ -457,16 +544,17 @@ __device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V
         const auto term_n = [&](const NbrState& n) {
             return A::template pair<kHLow>(P, pij, x, sub(v, vel_of(n.vq)), qi, n.vq.z, dens, n.vq.w);
         };
-        list_or_walk<G>(L, i, test_n, term_n, add_terms, fl,
-                        [&] { G::window(L.off + P.cbL, P.dimL[0], csx, cex, csy, cey, test, term, add_terms, fl); });
+        list_or_walk<G>(valid, L, i, test_n, term_n, add_terms, fl, [&](bool on) {
+            G::window(on, L.off + P.cbL, P.dimL[0], csx, cex, csy, cey, test, term, add_terms, fl);
+        });
     }
-    const float2 accB = wall_sum<A, G, 0>(P, V, p, csx, cex, csy, cey, P.Tle_r, P.cBL);
+    const float2 accB = wall_sum<A, G, 0>(valid, P, V, p, csx, cex, csy, cey, P.Tle_r, P.cBL);
     PairTerms fh{make_float2(0.f, 0.f), fl.t};  // (accH, accT): the sigma sum continues
     if (cross) {
         grid_coord_s<1>(P, p.x, p.y, -P.r, csx, csy);
         grid_coord_s<1>(P, p.x, p.y, P.r, cex, cey);
         G::window(
-            H.off + P.cbH, P.dimH[0], csx, cex, csy, cey,
+            valid, H.off + P.cbH, P.dimH[0], csx, cex, csy, cey,
             [&](int k) {
                 if (!lamLH(s, H.st[k])) return false;
                 pij = sub(p, H.pos[k]);
@@ -511,7 +599,7 @@ __device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V
     } else if (P.merge && s == 1u && !in_roi) {
         ns = 0;
     }
-    if (G::leader()) {
+    if (valid && G::leader()) {
         L.acc[i] = acc;
         if (!isfinite(acc.x) || !isfinite(acc.y)) atomicOr(&V.cnt->err, kErrNumeric);
         // a split parent's tether radius, 0.75 sqrt(m / (rho pi)) in double as the
@@ -541,10 +629,9 @@ __device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V
     return flag;
 }
 
-// One particle per thread: a warp-uniform loop (every lane makes the same number of
-// trips, lanes past n inactive) so the ballot that feeds the split compaction sees
-// whole warps; a warp's 32 particles lie in one compaction tile (kSplitTile % 32 ==
-// 0).  One particle per warp: the leader counts its particle's split.
+// A warp-uniform loop (every lane makes the same number of trips, lanes past n
+// inactive) so the ballot that feeds the split compaction sees whole warps; a warp's
+// particles lie in one compaction tile (kSplitTile % 32 == 0).
 // 48 registers (five blocks per SM) in both forms of the exact arithmetic.  The
 // batched form measured the same at 40 and 48 on a batch of 512 mixed scenes (4.11
 // / 4.08 ms), 3-7 % faster at 48 on batches of one scene, and 10 % slower at 64.
@@ -555,27 +642,33 @@ template <bool B, class G, class A>
 __global__ void __launch_bounds__(256, (A::kFast && !B) ? 6 : 5) k_force_low(Params P0, StepView V) {
     const int n = V.cnt->cur[0];
     const bool cross = V.cnt->h_state0 != 0, deleted = V.cnt->l_deleted != 0;
-    const auto one = [&](int i) {
-        if constexpr (B) {
-            const Params& P = V.table[V.scL[i]];
-            return force_low_one<A, G>(P, V, i, cross, deleted);
-        } else {
-            return force_low_one<A, G>(P0, V, i, cross, deleted);
-        }
-    };
-    if constexpr (G::kWarp) {
-        for_each_particle<G>(n, [&](int i) {
-            if (one(i) && G::leader()) atomicAdd(&V.split_tile[i / kSplitTile], 1u);
-        });
-    } else {
+    by_size<G, true>(n, [&](auto form, int) {
+        using F = decltype(form);
+        const auto one = [&](int i, bool valid) {
+            if constexpr (B) {
+                const Params& P = V.table[V.scL[i]];
+                return force_low_one<A, F>(P, V, i, valid, cross, deleted);
+            } else {
+                return force_low_one<A, F>(P0, V, i, valid, cross, deleted);
+            }
+        };
         const int lane = threadIdx.x & 31;
-        for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-            const int i = base + threadIdx.x;
-            const bool flag = i < n && one(i);
-            const unsigned m = __ballot_sync(0xffffffffu, flag);
-            if (lane == 0 && m) atomicAdd(&V.split_tile[(base + (threadIdx.x & ~31)) / kSplitTile], __popc(m));
+        if constexpr (F::kLanes > 1) {
+            for_each_particle<F>(n, [&](int i, bool valid) {
+                const bool flag = one(i, valid);
+                const unsigned m = __ballot_sync(0xffffffffu, flag && valid && F::leader());
+                // the warp's particles are neighbours; lane 0 has the first of them
+                if (lane == 0 && m) atomicAdd(&V.split_tile[i / kSplitTile], __popc(m));
+            });
+        } else {
+            for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+                const int i = base + threadIdx.x;
+                const bool flag = i < n && one(i, true);
+                const unsigned m = __ballot_sync(0xffffffffu, flag);
+                if (lane == 0 && m) atomicAdd(&V.split_tile[(base + (threadIdx.x & ~31)) / kSplitTile], __popc(m));
+            }
         }
-    }
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -585,7 +678,7 @@ __global__ void __launch_bounds__(256, (A::kFast && !B) ? 6 : 5) k_force_low(Par
 // low-res states are read after this step's split marks, as in the reference.
 // ---------------------------------------------------------------------------
 template <class A, class G>
-__device__ __forceinline__ void force_high_one(const Params& P, const StepView& V, int i) {
+__device__ __forceinline__ void force_high_one(const Params& P, const StepView& V, int i, bool valid) {
     const ScaleView& H = V.H;
     const ScaleView& L = V.L;
     const float4 own = H.vq[i];
@@ -617,8 +710,9 @@ __device__ __forceinline__ void force_high_one(const Params& P, const StepView& 
         const auto term_n = [&](const NbrState& n) {
             return A::template pair<kHHigh>(P, pij, x, sub(v, vel_of(n.vq)), qi, n.vq.z, dens, n.vq.w);
         };
-        list_or_walk<G>(H, i, test_n, term_n, add_terms, fh,
-                        [&] { G::window(H.off + P.cbH, P.dimH[0], csx, cex, csy, cey, test, term, add_terms, fh); });
+        list_or_walk<G>(valid, H, i, test_n, term_n, add_terms, fh, [&](bool on) {
+            G::window(on, H.off + P.cbH, P.dimH[0], csx, cex, csy, cey, test, term, add_terms, fh);
+        });
     }
     grid_coord_s<0>(P, p.x, p.y, -P.r, csx, csy);
     grid_coord_s<0>(P, p.x, p.y, P.r, cex, cey);
@@ -629,7 +723,7 @@ __device__ __forceinline__ void force_high_one(const Params& P, const StepView& 
     const bool odd = (s & 1u) != 0u;
     const uint8_t stamp = static_cast<uint8_t>(V.cnt->steps);
     G::window_if(
-        L.off + P.cbL, P.dimL[0], csx, cex, csy, cey,
+        valid, L.off + P.cbL, P.dimL[0], csx, cex, csy, cey,
         [&](int row) {
             if (!odd) return true;
             const uint8_t* f = L.cflag + P.cbL + row;
@@ -649,7 +743,7 @@ __device__ __forceinline__ void force_high_one(const Params& P, const StepView& 
             return A::template pair<kHCross>(P, pij, x, sub(v, vel_of(o)), qi, o.z, dens, o.w);
         },
         add_terms, fl);
-    const float2 accB = wall_sum<A, G, 1>(P, V, p, csx, cex, csy, cey, P.Tle_rh, P.cBH);
+    const float2 accB = wall_sum<A, G, 1>(valid, P, V, p, csx, cex, csy, cey, P.Tle_rh, P.cBH);
     float2 acc = fh.a, accL = fl.a;
     const float2 accT = fl.t;
     acc.x *= -P.mH;
@@ -687,7 +781,7 @@ __device__ __forceinline__ void force_high_one(const Params& P, const StepView& 
             }
         }
     }
-    if (!G::leader()) return;
+    if (!valid || !G::leader()) return;
     H.acc[i] = acc;
     if (!isfinite(acc.x) || !isfinite(acc.y)) atomicOr(&V.cnt->err, kErrNumeric);
     H.npos[i] = p;
@@ -720,13 +814,16 @@ __device__ __forceinline__ void force_high_one(const Params& P, const StepView& 
 // exact arithmetic's batched form was 8 % slower at five.
 template <bool B, class G, class A>
 __global__ void __launch_bounds__(256, B ? (A::kFast ? 5 : 4) : (A::kFast ? 6 : 5)) k_force_high(Params P0, StepView V) {
-    for_each_particle<G>(V.cnt->cur[1], [&](int i) {
-        if constexpr (B) {
-            const Params& P = V.table[V.scH[i]];
-            force_high_one<A, G>(P, V, i);
-        } else {
-            force_high_one<A, G>(P0, V, i);
-        }
+    by_size<G, true>(V.cnt->cur[1], [&](auto form, int n) {
+        using F = decltype(form);
+        for_each_particle<F>(n, [&](int i, bool valid) {
+            if constexpr (B) {
+                const Params& P = V.table[V.scH[i]];
+                force_high_one<A, F>(P, V, i, valid);
+            } else {
+                force_high_one<A, F>(P0, V, i, valid);
+            }
+        });
     });
 }
 

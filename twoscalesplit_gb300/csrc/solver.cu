@@ -104,10 +104,6 @@ cudaError_t tss_solver::mark(int k, cudaStream_t s) {
 cudaError_t tss_solver::enqueue_step(cudaStream_t s) {
     cudaError_t e;
     StepView V = view();
-    // the force passes read the neighbour lists their scale's density pass records
-    // when that pass runs one particle per thread
-    if (launch.per_warp[1]) V.L.nbr = nullptr;
-    if (launch.per_warp[0]) V.H.nbr = nullptr;
     // Outside profiling, the two grid builds and the two density passes each run as
     // two branches of the step graph: the low-res one on the side stream beside the
     // high-res one, joined before the first kernel that reads both (and the split
@@ -188,7 +184,12 @@ tss_status tss_solver::apply_launch(const tss_launch& l) {
         const bool low = g == 1 || g == 2;
         const long long lanes = l.per_warp[g] ? 32 : 1;  // threads per particle
         const long long cap = std::max(low ? nL : capH, 1) * lanes;
-        const long long cover = (cap + t - 1) / t;
+        // enough threads for a list that is short enough for groups of lanes (sph.cuh)
+        const bool force = g >= 2;
+        const auto group = [&](long long w, long long most) { return w * std::min(cap, most); };
+        const long long grouped = l.per_warp[g] ? 0 : std::max(group(8, force ? kForce8Max : kDensity8Max),
+                                                               force ? group(4, kForce4Max) : 0);
+        const long long cover = (std::max(cap, grouped) + t - 1) / t;
         if (l.persistent[g]) {
             const int occ = gather_occupancy(g, batched, l.per_warp[g] != 0, arith == TSS_ARITH_FAST, t);
             if (occ <= 0) return fail(TSS_CUDA_ERROR, "occupancy query of a gather kernel failed");

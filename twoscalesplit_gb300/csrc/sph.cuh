@@ -29,7 +29,7 @@ struct ScaleView {
     // nbr[c * nbr_stride + i] = j - i for its c-th same-scale neighbour within the
     // density's support (itself left out), in window order; nnbr[i] is their count,
     // kNbrOverflow when there are more than kMaxNbr or an offset does not fit 16
-    // bits.  Null when the density pass of this step did not record them.
+    // bits.
     int16_t* nbr;
     uint8_t* nnbr;
     long long nbr_stride;  // entries per list column: the scale's capacity
@@ -75,6 +75,21 @@ struct StepView {
 // growing: a grid build borrows the lists for its permutation (12 bytes an entry).
 constexpr int kMaxNbr = 24;
 constexpr uint8_t kNbrOverflow = 255;
+
+// Short lists: one particle per thread leaves most of the GPU idle and a step waits
+// for each thread's chain of loads and pairs.  A list of at most so many particles is
+// taken by groups of 8 or 4 lanes a particle (gather.cuh), whatever its capacity: the
+// kernels choose by the count on the device.  Stage times in us (n low-res and about
+// as many high-res particles; exact arithmetic; one thread / 4 / 8 / 16 lanes):
+//   n          1,500              10,000             22,000             48,000
+//   low force  24 / 16 / 14 / 12  24 / 17 / 14 / 14  24 / 18 / 16 / 20  24 / 18 / 24 / 30
+//   high force 31 / 21 / 16 / 15  28 / 20 / 17 / 18  28 / 21 / 19 / 25  33 / 26 / 29 / 38
+//   low dens.  11 / 11 / 11 / 9   11 / 13 / 11 / 11  12 / 13 / 14 / 17  13 / 17 / 21 / 25
+//   high dens. 12 / 11 / 10 / 8   12 / 12 / 10 / 12  12 / 13 / 14 / 16  17 / 17 / 20 / 26
+// A density search is short and its groups do more work than its threads (the two run
+// as parallel branches), so it returns to one thread earlier than a force does.
+constexpr int kDensity8Max = 12000;
+constexpr int kForce8Max = 20000, kForce4Max = 48000;
 
 constexpr int kSplitThreads = 256;
 constexpr int kSplitItems = 16;
