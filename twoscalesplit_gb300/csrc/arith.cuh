@@ -31,19 +31,9 @@
 
 namespace tss {
 
-__device__ __forceinline__ float rsqrt_approx(float x) {
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 __device__ __forceinline__ float sqrt_approx(float x) {
     float y;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float rcp_approx(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 
@@ -58,6 +48,11 @@ struct ExactArith {
     __device__ __forceinline__ static PairTerms pair(const Params& P, float2 pij, float x, float2 vij, float qi,
                                                      float qj, float densi, float densj) {
         const float h = HS == kHLow ? P.r : (HS == kHCross ? P.hx : P.rh);
+        const float2 vp = mul2(vij, pij);
+        const float dvp = vp.x + vp.y;
+        const float dsum = densi + densj;
+        if (pair_in_range(P, x, dvp, dsum))
+            return pair_terms_in_range<HS == kHHigh>(P, pij, x, dvp, qi, qj, dsum, h);
         return pair_terms(P, pij, sqrtf(x), vij, qi, qj, densi, densj, h);
     }
 

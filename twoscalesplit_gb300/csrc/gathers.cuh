@@ -523,9 +523,7 @@ __device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V
     PairTerms fl{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};  // (acc, accT)
     float2 pij = make_float2(0.f, 0.f);
     float x = 0.0f;
-    int csx, csy, cex, cey;
-    grid_coord_s<0>(P, p.x, p.y, -P.r, csx, csy);
-    grid_coord_s<0>(P, p.x, p.y, P.r, cex, cey);
+    int csx, csy, cex, cey;  // found where they are used: few values live through the list loop
     {
         const auto test = [&](int k) {
             pij = sub(p, L.pos[k]);
@@ -545,9 +543,13 @@ __device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V
             return A::template pair<kHLow>(P, pij, x, sub(v, vel_of(n.vq)), qi, n.vq.z, dens, n.vq.w);
         };
         list_or_walk<G>(valid, L, i, test_n, term_n, add_terms, fl, [&](bool on) {
+            grid_coord_s<0>(P, p.x, p.y, -P.r, csx, csy);
+            grid_coord_s<0>(P, p.x, p.y, P.r, cex, cey);
             G::window(on, L.off + P.cbL, P.dimL[0], csx, cex, csy, cey, test, term, add_terms, fl);
         });
     }
+    grid_coord_s<0>(P, p.x, p.y, -P.r, csx, csy);
+    grid_coord_s<0>(P, p.x, p.y, P.r, cex, cey);
     const float2 accB = wall_sum<A, G, 0>(valid, P, V, p, csx, cex, csy, cey, P.Tle_r, P.cBL);
     PairTerms fh{make_float2(0.f, 0.f), fl.t};  // (accH, accT): the sigma sum continues
     if (cross) {
@@ -689,8 +691,6 @@ __device__ __forceinline__ void force_high_one(const Params& P, const StepView& 
     float2 pij = make_float2(0.f, 0.f);
     float x = 0.0f;
     int csx, csy, cex, cey;
-    grid_coord_s<1>(P, p.x, p.y, -P.rh, csx, csy);
-    grid_coord_s<1>(P, p.x, p.y, P.rh, cex, cey);
     {
         const auto test = [&](int k) {
             if (!lamHH(s, H.st[k])) return false;
@@ -711,6 +711,8 @@ __device__ __forceinline__ void force_high_one(const Params& P, const StepView& 
             return A::template pair<kHHigh>(P, pij, x, sub(v, vel_of(n.vq)), qi, n.vq.z, dens, n.vq.w);
         };
         list_or_walk<G>(valid, H, i, test_n, term_n, add_terms, fh, [&](bool on) {
+            grid_coord_s<1>(P, p.x, p.y, -P.rh, csx, csy);
+            grid_coord_s<1>(P, p.x, p.y, P.rh, cex, cey);
             G::window(on, H.off + P.cbH, P.dimH[0], csx, cex, csy, cey, test, term, add_terms, fh);
         });
     }

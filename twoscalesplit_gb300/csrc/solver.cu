@@ -399,6 +399,7 @@ Params make_params(const SceneIn& sc) {
     }
     P.fEps = make_float3(eps[0], eps[1], eps[2]);
     P.fKv = make_float3(kv[0], kv[1], kv[2]);
+    P.safe = pair_safe(P) ? 1 : 0;
     P.fKw = static_cast<float>(0.02 * static_cast<double>(cfg->speed_sound) * cfg->speed_sound);
     return P;
 }
