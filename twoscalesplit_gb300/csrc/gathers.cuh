@@ -456,6 +456,8 @@ __global__ void __launch_bounds__(256, B ? 6 : 8) k_density_low(Params P0, StepV
     __shared__ int16_t s_nbr[G::kLanes > 1 ? 1 : kNbrRows * kNbrCols];
     int16_t* const nbr_col = s_nbr + (G::kLanes > 1 ? 0 : threadIdx.x);
     const bool cross = V.cnt->h_state0 != 0;
+    // the split counts of the low-res force's tiles, zero before it
+    for (int t = tid(); t < (V.cnt->cur[0] + kSplitTile - 1) / kSplitTile; t += nthreads()) V.split_tile[t] = 0u;
     by_size<G, false>(V.cnt->cur[0], [&](auto form, int n) {
         using F = decltype(form);
         for_each_particle<F>(n, [&](int i, bool valid) {
@@ -642,6 +644,7 @@ __device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V
 // (0.130 -> 0.125 ms); batched, it would spill 76 bytes at 40 and keeps 48.
 template <bool B, class G, class A>
 __global__ void __launch_bounds__(256, (A::kFast && !B) ? 6 : 5) k_force_low(Params P0, StepView V) {
+    let_next_start();
     const int n = V.cnt->cur[0];
     const bool cross = V.cnt->h_state0 != 0, deleted = V.cnt->l_deleted != 0;
     by_size<G, true>(n, [&](auto form, int) {
@@ -716,6 +719,9 @@ __device__ __forceinline__ void force_high_one(const Params& P, const StepView& 
             G::window(on, H.off + P.cbH, P.dimH[0], csx, cex, csy, cey, test, term, add_terms, fh);
         });
     }
+    // up to here, the high-res list alone: this kernel starts while the low-res force's
+    // last blocks run.  From here, what the low-res force wrote
+    wait_for_previous();
     grid_coord_s<0>(P, p.x, p.y, -P.r, csx, csy);
     grid_coord_s<0>(P, p.x, p.y, P.r, cex, cey);
     PairTerms fl{make_float2(0.f, 0.f), fh.t};  // (accL, accT): the sigma sum continues
@@ -846,7 +852,7 @@ void launch_gather_bg(int g, int blocks, int threads, cudaStream_t s, const Para
             k_force_low<B, G, A><<<blocks, threads, 0, s>>>(P, V);
             break;
         case 3:
-            k_force_high<B, G, A><<<blocks, threads, 0, s>>>(P, V);
+            launch_after(k_force_high<B, G, A>, blocks, threads, s, P, V);
             break;
         default:
             break;

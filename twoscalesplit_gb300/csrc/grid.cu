@@ -39,6 +39,7 @@ __global__ void k_grid_keys(const float2* __restrict__ pos, const int* __restric
 // sized for its capacity); counts are zeroed for the next key pass (only the
 // 16-byte groups that hold a non-zero count are written back).
 __global__ void __launch_bounds__(kScanThreads) k_grid_scan(GridBufs g) {
+    let_next_start();
     __shared__ unsigned s_warp[kScanThreads / 32];
     __shared__ unsigned s_red[kScanThreads / 32];
     const int C = g.used ? min(*g.used, g.ncells) : g.ncells;
@@ -151,6 +152,8 @@ __global__ void __launch_bounds__(kScanThreads) k_grid_scan(GridBufs g) {
 // skips those entries instead of touching memory outside its buffers.
 __global__ void k_grid_scatter(const int* __restrict__ n_ptr, const int32_t* __restrict__ id, GridBufs g,
                                unsigned* err) {
+    let_next_start();
+    wait_for_previous();
     const int n = *n_ptr;
     const int total = *g.total;
     if (blockIdx.x == 0 && threadIdx.x == 0) {  // the scan's list of big cells, for the reorder
@@ -300,8 +303,12 @@ __device__ __forceinline__ int lower_rank(const int* __restrict__ sorted, int k,
 // the bigger cells (listed by the scan) are placed whole by one block each.
 __global__ void __launch_bounds__(kReorderThreads) k_grid_reorder(int* n_ptr, int cap, GridBufs g, ReorderArgs a,
                                                                   unsigned* err) {
+    wait_for_previous();
     const int n = *g.total;
     if (blockIdx.x == 0 && threadIdx.x == 0) *n_ptr = n;
+    // the tile sums, zero for the next key pass
+    const int tiles = ((g.used ? min(*g.used, g.ncells) : g.ncells) + kScanTile - 1) / kScanTile;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < tiles; t += gridDim.x * blockDim.x) g.tile_sum[t] = 0u;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         int2 pe = g.perm[k];
         const int src = pe.x, id = pe.y;
@@ -420,12 +427,10 @@ cudaError_t grid_sort_enqueue(const int32_t* id, int* n_ptr, int cap, GridBufs g
     const int T = 256;
     const int pb = particle_blocks(cap, T);
     const int sb = g.ntiles < 8 * sm_count() ? g.ntiles : 8 * sm_count();
-    cudaError_t e;
     k_grid_scan<<<sb, kScanThreads, 0, stream>>>(g);
-    if ((e = cudaMemsetAsync(g.tile_sum, 0, sizeof(unsigned) * g.ntiles, stream)) != cudaSuccess) return e;
-    k_grid_scatter<<<pb, T, 0, stream>>>(n_ptr, id, g, err);
-    k_grid_reorder<<<pb, kReorderThreads, 0, stream>>>(n_ptr, cap, g, a, err);
-    return cudaGetLastError();
+    cudaError_t e = launch_after(k_grid_scatter, pb, T, stream, n_ptr, id, g, err);
+    if (e == cudaSuccess) e = launch_after(k_grid_reorder, pb, kReorderThreads, stream, n_ptr, cap, g, a, err);
+    return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 cudaError_t grid_build_enqueue(const float2* pos, const int32_t* id, int* n_ptr, int cap, float ox, float oy,

@@ -134,9 +134,7 @@ cudaError_t tss_solver::enqueue_step(cudaStream_t s) {
     if (branch && (e = join()) != cudaSuccess) return e;
     // 2. relaxation of last step's children (older snapshot's relaxTransient)
     for (int it = 0; it < P.relax_iters; ++it) {
-        launch_k_relax_density(batched, blocksH, 256, s, P, V);
-        launch_k_relax_force(batched, blocksH, 256, s, P, V);
-        k_relax_apply<<<blocksH, 256, 0, s>>>(P, V);
+        if ((e = launch_relax(batched, blocksH, 256, s, P, V)) != cudaSuccess) return e;
     }
     if ((e = mark(3, s)) != cudaSuccess) return e;
     // 3. densities, 4. low force + advance + split marks, 5. children, 6. high force
@@ -150,7 +148,6 @@ cudaError_t tss_solver::enqueue_step(cudaStream_t s) {
     gather(1, sl);
     if ((e = mark(5, s)) != cudaSuccess) return e;
     if (branch && (e = join()) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(split_tile, 0, sizeof(unsigned) * split_ntiles, s)) != cudaSuccess) return e;
     gather(2, s);
     if ((e = mark(6, s)) != cudaSuccess) return e;
     // The split compaction appends children past the high-res list that the

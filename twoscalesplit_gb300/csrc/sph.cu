@@ -173,6 +173,8 @@ __device__ __forceinline__ void relax_density_one(const Params& P, const StepVie
 
 template <bool B>
 __global__ void __launch_bounds__(256) k_relax_density(Params P0, StepView V) {
+    let_next_start();
+    wait_for_previous();
     const int nf = min(4 * V.cnt->n_fresh, P0.capH);  // relaxation scratch holds capH entries
     for (int f = tid(); f < nf; f += nthreads()) {
         const int i = fresh_child(P0, V, f);
@@ -257,6 +259,8 @@ __device__ __forceinline__ void relax_force_one(const Params& P, const StepView&
 
 template <bool B>
 __global__ void __launch_bounds__(256) k_relax_force(Params P0, StepView V) {
+    let_next_start();
+    wait_for_previous();
     const int nf = min(4 * V.cnt->n_fresh, P0.capH);  // relaxation scratch holds capH entries
     for (int f = tid(); f < nf; f += nthreads()) {
         const int i = fresh_child(P0, V, f);
@@ -271,6 +275,8 @@ __global__ void __launch_bounds__(256) k_relax_force(Params P0, StepView V) {
 }
 
 __global__ void k_relax_apply(Params P0, StepView V) {
+    let_next_start();
+    wait_for_previous();
     const int nf = min(4 * V.cnt->n_fresh, P0.capH);  // relaxation scratch holds capH entries
     for (int f = tid(); f < nf; f += nthreads()) {
         const int i = fresh_child(P0, V, f);
@@ -340,17 +346,19 @@ void launch_wall_near(const int* woff, uint8_t* wnear, int dimx, int dimy, cudaS
     k_wall_near<<<blocks, 256, 0, s>>>(woff, wnear, dimx, dimy);
 }
 
-#define TSS_LAUNCHER(NAME)                                                                        \
-    void launch_##NAME(bool batched, int blocks, int threads, cudaStream_t s, const Params& P,   \
-                       const StepView& V) {                                                       \
-        if (batched)                                                                              \
-            NAME<true><<<blocks, threads, 0, s>>>(P, V);                                          \
-        else                                                                                      \
-            NAME<false><<<blocks, threads, 0, s>>>(P, V);                                         \
-    }
-TSS_LAUNCHER(k_split)
-TSS_LAUNCHER(k_relax_density)
-TSS_LAUNCHER(k_relax_force)
-#undef TSS_LAUNCHER
+void launch_k_split(bool batched, int blocks, int threads, cudaStream_t s, const Params& P, const StepView& V) {
+    if (batched)
+        k_split<true><<<blocks, threads, 0, s>>>(P, V);
+    else
+        k_split<false><<<blocks, threads, 0, s>>>(P, V);
+}
+
+cudaError_t launch_relax(bool batched, int blocks, int threads, cudaStream_t s, const Params& P, const StepView& V) {
+    cudaError_t e = launch_after(batched ? k_relax_density<true> : k_relax_density<false>, blocks, threads, s, P, V);
+    if (e == cudaSuccess)
+        e = launch_after(batched ? k_relax_force<true> : k_relax_force<false>, blocks, threads, s, P, V);
+    if (e == cudaSuccess) e = launch_after(k_relax_apply, blocks, threads, s, P, V);
+    return e;
+}
 
 }  // namespace tss

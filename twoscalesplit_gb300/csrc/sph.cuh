@@ -112,8 +112,8 @@ __global__ void k_step_finish(Counters* c);
 void launch_gather(int g, bool batched, bool warp, bool fast, int blocks, int threads, cudaStream_t s,
                    const Params& P, const StepView& V);
 void launch_k_split(bool batched, int blocks, int threads, cudaStream_t s, const Params& P, const StepView& V);
-void launch_k_relax_density(bool batched, int blocks, int threads, cudaStream_t s, const Params& P, const StepView& V);
-void launch_k_relax_force(bool batched, int blocks, int threads, cudaStream_t s, const Params& P, const StepView& V);
+// one relaxation sub-step: density, force, apply
+cudaError_t launch_relax(bool batched, int blocks, int threads, cudaStream_t s, const Params& P, const StepView& V);
 // resident blocks per SM of gather g at `threads` threads per block; 0 on error
 int gather_occupancy(int g, bool batched, bool warp, bool fast, int threads);
 // wnear of one scene's dimx x dimy low grid from its wall cell offsets (both
