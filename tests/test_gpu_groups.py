@@ -58,3 +58,20 @@ def test_list_lengths(n_low, n_high, q1):
             assert np.array_equal(d["id"], st["id"]) and np.array_equal(d["state"], st["state"]), (k, s)
             for f in ("pos", "vel"):
                 assert np.array_equal(d[f], st[f].astype(np.float32), equal_nan=True), (k, s, f)
+
+
+@pytest.mark.parametrize("nx", [3, 40, 80])
+def test_relaxing_few_and_many_children(nx):
+    # 4 nx^2 children relax at once: by groups of lanes, or (25,600) one per thread
+    sc = scenes.dam_break_small(nx, nx, dx=0.4 / nx, seed=nx, relax_iters=2, roi=[-1.0, -1.0, 2.0, 2.0])
+    sc.config.flags |= _abi.TSS_FLAG_OLDER_PLACEMENT
+    sol, orc = Solver.from_scene(sc), O.Oracle(sc, 32)
+    for k in range(3):
+        sol.step(1)
+        orc.step()
+        for s in (0, 1):
+            d, st = sol.download(s), orc.state(s)
+            assert np.array_equal(d["id"], st["id"]), (k, s)
+            for f in ("pos", "vel"):
+                assert np.array_equal(d[f], st[f].astype(np.float32), equal_nan=True), (k, s, f)
+    assert sol.counts()["n_high"] == 4 * nx * nx

@@ -136,37 +136,43 @@ __device__ __forceinline__ int fresh_child(const Params& P0, const StepView& V, 
     return (slot >= 0 && slot < P0.slotsH) ? V.H.map[slot] : -1;
 }
 
-__device__ __forceinline__ void relax_density_one(const Params& P, const StepView& V, int i) {
+// f(form, child f, valid) over the nf children created in the last step: a group of
+// eight lanes a child unless they are many.  They are usually few, and the kernels wait
+// for one child's chain of candidates: four sub-steps of a 5,000-particle scene took 59
+// us with a thread a child and take 36.
+template <class F>
+__device__ __forceinline__ void for_each_fresh(int nf, F&& f) {
+    by_size<PerThread, false>(nf, [&](auto form, int n) {
+        for_each_particle<decltype(form)>(n, [&](int k, bool valid) { f(form, k, valid); });
+    });
+}
+
+template <class G>
+__device__ __forceinline__ void relax_density_one(const Params& P, const StepView& V, int i, bool on) {
     const ScaleView& H = V.H;
     const ScaleView& L = V.L;
-    const int* offH = H.off + P.cbH;
-    const int* offL = L.off + P.cbL;
     const float2 p = H.pos[i];
-    float d = 0.0f, dl = 0.0f;
+    float d = 0.0f, dl = 0.0f, dist = 0.0f;
     int csx, csy, cex, cey;
+    const auto sum = [&](const ScaleView& X, int cb, int dimx, float& into) {
+        G::window(
+            on, X.off + cb, dimx, csx, cex, csy, cey,
+            [&](int j) {
+                dist = vnorm(sub(p, X.pos[j]));
+                return dist <= P.rh;
+            },
+            [&](int) { return kernW(dist, P.rh, P.CH); }, add_density, into);
+    };
     grid_coord_s<1>(P, p.x, p.y, -P.rh, csx, csy);
     grid_coord_s<1>(P, p.x, p.y, P.rh, cex, cey);
-    for (int cy = csy; cy <= cey; ++cy) {
-        const int row = cy * P.dimH[0];
-        const int b = offH[row + cex + 1];
-        for (int j = offH[row + csx]; j < b; ++j) {
-            float dist = vnorm(sub(p, H.pos[j]));
-            if (dist <= P.rh) d += kernW(dist, P.rh, P.CH);
-        }
-    }
+    sum(H, P.cbH, P.dimH[0], d);
     grid_coord_s<0>(P, p.x, p.y, -P.rh, csx, csy);
     grid_coord_s<0>(P, p.x, p.y, P.rh, cex, cey);
-    for (int cy = csy; cy <= cey; ++cy) {
-        const int row = cy * P.dimL[0];
-        const int b = offL[row + cex + 1];
-        for (int j = offL[row + csx]; j < b; ++j) {
-            float dist = vnorm(sub(p, L.pos[j]));
-            if (dist <= P.rh) dl += kernW(dist, P.rh, P.CH);
-        }
-    }
+    sum(L, P.cbL, P.dimL[0], dl);
     d *= P.mH;
     dl *= P.mL;
     d += dl;
+    if (!on || !G::leader()) return;
     H.dens[i] = d;
     H.pres[i] = tait(d, P);
 }
@@ -176,71 +182,58 @@ __global__ void __launch_bounds__(256) k_relax_density(Params P0, StepView V) {
     let_next_start();
     wait_for_previous();
     const int nf = min(4 * V.cnt->n_fresh, P0.capH);  // relaxation scratch holds capH entries
-    for (int f = tid(); f < nf; f += nthreads()) {
-        const int i = fresh_child(P0, V, f);
-        if (i < 0) continue;
-        if constexpr (B) {
-            const Params& P = V.table[V.scH[i]];
-            relax_density_one(P, V, i);
-        } else {
-            relax_density_one(P0, V, i);
-        }
-    }
+    for_each_fresh(nf, [&](auto form, int f, bool valid) {
+        const int c = fresh_child(P0, V, f), i = max(c, 0);
+        relax_density_one<decltype(form)>(B ? V.table[V.scH[i]] : P0, V, i, valid && c >= 0);
+    });
 }
 
-__device__ __forceinline__ void relax_force_one(const Params& P, const StepView& V, int i, int f) {
+template <class G>
+__device__ __forceinline__ void relax_force_one(const Params& P, const StepView& V, int i, int f, bool on) {
     const ScaleView& H = V.H;
     const ScaleView& L = V.L;
-    const int* offH = H.off + P.cbH;
-    const int* offL = L.off + P.cbL;
-    const int* woff = V.woff + P.cbL;
     const float2* wpos = V.wpos + P.wb;
     float2 p = H.pos[i], v = vel_of(H.vq[i]);
     const float dens = H.dens[i], pre = H.pres[i];
     const float dens2 = dens * dens;
     float2 acc = make_float2(0.f, 0.f), accL = make_float2(0.f, 0.f), accB = make_float2(0.f, 0.f);
+    float2 x = make_float2(0.f, 0.f);
+    float dist = 0.0f;
+    const auto add = [](float2& a, float2 t) {
+        a.x += t.x;
+        a.y += t.y;
+    };
     int csx, csy, cex, cey;
+    const auto sum = [&](const ScaleView& X, int cb, int dimx, float2& into) {
+        G::window(
+            on, X.off + cb, dimx, csx, cex, csy, cey,
+            [&](int j) {
+                x = sub(p, X.pos[j]);
+                dist = vnorm(x);
+                return dist != 0.0f && dist < P.rh;
+            },
+            [&](int j) {
+                const float dj = X.dens[j];
+                const float coeff = pre / dens2 + X.pres[j] / (dj * dj);
+                const float2 g = kernDW(x, dist, P.rh, P.GH);
+                return make_float2(coeff * g.x, coeff * g.y);
+            },
+            add, into);
+    };
     grid_coord_s<1>(P, p.x, p.y, -P.rh, csx, csy);
     grid_coord_s<1>(P, p.x, p.y, P.rh, cex, cey);
-    for (int cy = csy; cy <= cey; ++cy) {
-        const int row = cy * P.dimH[0];
-        const int b = offH[row + cex + 1];
-        for (int j = offH[row + csx]; j < b; ++j) {
-            const float2 pij = sub(p, H.pos[j]);
-            const float dist = vnorm(pij);
-            if (dist != 0.0f && dist < P.rh) {
-                const float dj = H.dens[j];
-                const float coeff = pre / dens2 + H.pres[j] / (dj * dj);
-                const float2 g = kernDW(pij, dist, P.rh, P.GH);
-                acc.x += coeff * g.x;
-                acc.y += coeff * g.y;
-            }
-        }
-    }
+    sum(H, P.cbH, P.dimH[0], acc);
     grid_coord_s<0>(P, p.x, p.y, -P.rh, csx, csy);
     grid_coord_s<0>(P, p.x, p.y, P.rh, cex, cey);
-    for (int cy = csy; cy <= cey; ++cy) {
-        const int row = cy * P.dimL[0];
-        const int b = offL[row + cex + 1];
-        for (int j = offL[row + csx]; j < b; ++j) {
-            const float2 pij = sub(p, L.pos[j]);
-            const float dist = vnorm(pij);
-            if (dist != 0.0f && dist < P.rh) {
-                const float dj = L.dens[j];
-                const float coeff = pre / dens2 + L.pres[j] / (dj * dj);
-                const float2 g = kernDW(pij, dist, P.rh, P.GH);
-                accL.x += coeff * g.x;
-                accL.y += coeff * g.y;
-            }
-        }
-        const int wb = woff[row + cex + 1];
-        for (int k = woff[row + csx]; k < wb; ++k) {
+    sum(L, P.cbL, P.dimL[0], accL);
+    G::window(
+        on, V.woff + P.cbL, P.dimL[0], csx, cex, csy, cey, [](int) { return true; },
+        [&](int k) {
             const float2 pik = sub(p, wpos[k]);
             const float gm = wall_weight(vnorm(pik), P.rh, P.cs);
-            accB.x += P.cBH * gm * pik.x;
-            accB.y += P.cBH * gm * pik.y;
-        }
-    }
+            return make_float2(P.cBH * gm * pik.x, P.cBH * gm * pik.y);
+        },
+        add, accB);
     acc.x *= -P.mH;
     acc.y *= -P.mH;
     accL.x *= -P.mL;
@@ -253,6 +246,7 @@ __device__ __forceinline__ void relax_force_one(const Params& P, const StepView&
     v.y += P.relax_dt * acc.y;
     p.x += P.relax_dt * v.x;
     p.y += P.relax_dt * v.y;
+    if (!on || !G::leader()) return;
     V.relax_pos[f] = p;
     V.relax_vel[f] = v;
 }
@@ -262,16 +256,10 @@ __global__ void __launch_bounds__(256) k_relax_force(Params P0, StepView V) {
     let_next_start();
     wait_for_previous();
     const int nf = min(4 * V.cnt->n_fresh, P0.capH);  // relaxation scratch holds capH entries
-    for (int f = tid(); f < nf; f += nthreads()) {
-        const int i = fresh_child(P0, V, f);
-        if (i < 0) continue;
-        if constexpr (B) {
-            const Params& P = V.table[V.scH[i]];
-            relax_force_one(P, V, i, f);
-        } else {
-            relax_force_one(P0, V, i, f);
-        }
-    }
+    for_each_fresh(nf, [&](auto form, int f, bool valid) {
+        const int c = fresh_child(P0, V, f), i = max(c, 0);
+        relax_force_one<decltype(form)>(B ? V.table[V.scH[i]] : P0, V, i, f, valid && c >= 0);
+    });
 }
 
 __global__ void k_relax_apply(Params P0, StepView V) {
