@@ -60,6 +60,40 @@ def test_list_lengths(n_low, n_high, q1):
                 assert np.array_equal(d[f], st[f].astype(np.float32), equal_nan=True), (k, s, f)
 
 
+@pytest.mark.parametrize("cells", [500, 140000])
+def test_walls_of_wide_grids(cells):
+    # a grid of more columns than the two-cell rule for wall windows is used for; the
+    # particles stand on walls in its corners and outside it
+    rng = np.random.default_rng(cells)
+    r = 1.0 / cells
+    dx = 0.5 * r
+    cfg = _abi.config_init(0.0, 0.0, 1.0, 6 * r, r, dx, scenes.REST_DENSITY, scenes.TAIT_B, scenes.SPEED_SOUND,
+                           scenes.ALPHA, scenes.SIGMA, 1e-9)
+    cfg.roi[:] = [9.0, 9.0, 10.0, 10.0]
+    x = np.concatenate([np.arange(20) * dx, 1.0 - np.arange(1, 21) * dx, 0.5 + np.arange(20) * dx])
+    walls = np.stack([np.repeat(x, 2), np.tile([0.0, 0.5 * dx], len(x))], axis=1)
+    pos = np.stack([np.repeat(x, 5), np.tile(1.5 * dx + np.arange(5) * dx, len(x))], axis=1)
+    pos += rng.uniform(-0.2 * dx, 0.2 * dx, size=pos.shape)
+    pos[::37] += [[-4 * r, -5 * r]]
+    n = len(pos)
+    pos, vel = pos.astype(np.float32), rng.standard_normal((n, 2)).astype(np.float32)
+    m = scenes.REST_DENSITY * dx * dx
+    sc = scenes.Scene("wide", cfg, pos, vel, m, m / 4, 4 * n, walls.astype(np.float32), m / 4, 1, dx)
+    high = {"id": np.arange(4 * n, dtype=np.int32), "pos": (np.repeat(pos, 4, axis=0) + rng.uniform(-0.3 * dx, 0.3 * dx, size=(4 * n, 2))).astype(np.float32),
+            "vel": np.repeat(vel, 4, axis=0), "state": np.ones(4 * n, np.uint8)}
+    ids = np.arange(n, dtype=np.int32)
+    sol, orc = Solver.from_scene(sc), O.Oracle(sc, 32)
+    sol.upload(0, {"id": ids, "pos": pos, "vel": vel, "state": np.ones(n, np.uint8)})
+    orc.set_scale(0, ids, pos, vel, np.ones(n, np.uint8))
+    sol.upload(1, high)
+    orc.set_scale(1, high["id"], high["pos"], high["vel"], high["state"])
+    sol.step(1)
+    orc.step()
+    for s in (0, 1):
+        assert np.array_equal(sol.copy(s, _abi.TSS_BUF_SORTED_ID), orc.get(s, "sorted_id")), s
+        assert np.array_equal(sol.copy(s, _abi.TSS_BUF_ACCEL), orc.get(s, "acc").astype(np.float32), equal_nan=True), s
+
+
 @pytest.mark.parametrize("nx", [3, 40, 80])
 def test_relaxing_few_and_many_children(nx):
     # 4 nx^2 children relax at once: by groups of lanes, or (25,600) one per thread

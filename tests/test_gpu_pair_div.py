@@ -1,6 +1,6 @@
 """The square root, reciprocals and quotients of the force pairs in the exact arithmetic
-(tss_device.cuh) against the IEEE operations, bit for bit, and whole steps on both sides
-of the operand ranges where they hand over to those."""
+(tss_device.cuh) against the IEEE operations, and the tether radius against its FP64
+expression, bit for bit; whole steps on both sides of the pairs' operand ranges."""
 import os
 import subprocess
 
@@ -15,10 +15,11 @@ pytestmark = pytest.mark.gpu
 HERE = os.path.dirname(os.path.abspath(__file__))
 
 
-def test_quotients_equal_ieee_division(tmp_path):
+@pytest.mark.parametrize("probe", ["div_pair", "tether"])
+def test_equal_to_the_plain_expressions(tmp_path, probe):
     build.build()
-    exe = str(tmp_path / "div_pair")
-    subprocess.check_call([build.nvcc(), *build.flags(), os.path.join(HERE, "cuda", "div_pair.cu"), "-o", exe])
+    exe = str(tmp_path / probe)
+    subprocess.check_call([build.nvcc(), *build.flags(), os.path.join(HERE, "cuda", probe + ".cu"), "-o", exe])
     out = subprocess.check_output([exe], timeout=300).decode()
     assert out.strip().splitlines()[-1].startswith("mismatches 0 of"), out
 

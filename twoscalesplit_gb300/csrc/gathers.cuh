@@ -40,17 +40,23 @@ __device__ __forceinline__ void add_density(float& d, float t) { d += t; }
 // (PerGroup, every lane of a group taking the same particle).  f(i, valid): the
 // groups of a warp come together, those past the end with the last particle and
 // valid = false.
+// Taken by `blocks` blocks, of which this one is the `block`-th.
 template <class G, class F>
-__device__ __forceinline__ void for_each_particle(int n, F&& f) {
+__device__ __forceinline__ void for_each_particle(int n, int block, int blocks, F&& f) {
+    const int t0 = block * blockDim.x + threadIdx.x, step = blocks * blockDim.x;
     if constexpr (G::kLanes > 1) {
         constexpr int per = 32 / G::kLanes;  // particles per warp
-        for (int base = (tid() >> 5) * per; base < n; base += (nthreads() >> 5) * per) {
+        for (int base = (t0 >> 5) * per; base < n; base += (step >> 5) * per) {
             const int i = base + (static_cast<int>(threadIdx.x) & 31) / G::kLanes;
             f(min(i, n - 1), i < n);
         }
     } else {
-        for (int i = tid(); i < n; i += nthreads()) f(i, true);
+        for (int i = t0; i < n; i += step) f(i, true);
     }
+}
+template <class G, class F>
+__device__ __forceinline__ void for_each_particle(int n, F&& f) {
+    for_each_particle<G>(n, blockIdx.x, gridDim.x, f);
 }
 
 // f(form, n) with the form that takes n particles: the launch's own, except that one
@@ -410,6 +416,76 @@ __global__ void __launch_bounds__(256, B ? (A::kFast ? 6 : 5) : (A::kFast ? 8 : 
 }
 
 // ---------------------------------------------------------------------------
+// Wall term of a force sum (updateAccCell 562-579 / updateAccCellComplementHigh
+// 867-884): every wall particle of the window's cells, in cell order.  Pairs with
+// sqrtf(x) > rad have q >= 2 and add exactly zero, so they are skipped.  S selects
+// the scale: 0 the low-res radius r, 1 the high-res radius rh.  `cell`: the particle's
+// cell of the low-res grid.
+// ---------------------------------------------------------------------------
+template <class A, class G, int S>
+__device__ __forceinline__ float2 wall_sum(bool on, const Params& P, const StepView& V, float2 p, int cell) {
+    float2 accB = make_float2(0.f, 0.f);
+    // the window reaches at most two cells from the particle's own (near_cells): with no
+    // wall particle within two cells of that, the sum is empty
+    on = on && (!P.near_cells || V.wnear[P.cbL + cell]);
+    if (!G::any(on)) return accB;
+    int csx, csy, cex, cey;
+    grid_coord_s<0>(P, p.x, p.y, -P.r, csx, csy);
+    grid_coord_s<0>(P, p.x, p.y, P.r, cex, cey);
+    const float Tle = S ? P.Tle_rh : P.Tle_r, cB = S ? P.cBH : P.cBL;
+    const float2* wpos = V.wpos + P.wb;
+    float2 pik = make_float2(0.f, 0.f);
+    float x = 0.0f;
+    G::window(
+        on, V.woff + P.cbL, P.dimL[0], csx, cex, csy, cey,
+        [&](int k) {
+            pik = sub(p, wpos[k]);
+            x = sq(pik);
+            return !(x > Tle);  // NaN passes: the reference's 0 * NaN offset propagates it
+        },
+        [&](int) { return A::template wall<S>(P, pik, x, cB); },
+        [](float2& a, float2 t) {
+            a.x += t.x;
+            a.y += t.y;
+        },
+        accB);
+    return accB;
+}
+
+// The wall terms of lists short enough for groups of lanes.  They need the positions
+// alone, so blocks of their own take them in the low-res density's launch, and the force
+// reads them (acc holds them until it writes the accelerations).  A particle near a wall
+// has some 36 candidates and 20 pairs there, and a short list's step waits for it.
+// A step took, with the tether radius out of FP64 too, 37.2 -> 34.8 us at 5,000
+// particles (34.8 -> 31.9 us a step of a graph of eight), 43.6 -> 39.6 us at 22,000
+// (tolerance arithmetic).  A long list's step hides its walls' warps; taken here they
+// made one of 1.0M low-res particles slower (180 -> 183 us), as did a launch of their
+// own beside the densities for the steps of graphs of several (34.4 -> 36.4 us).
+template <bool B, class A, int S>
+__device__ __forceinline__ void wall_scale(const Params& P0, const StepView& V, const ScaleView& X, const uint16_t* sc,
+                                           int block, int blocks) {
+    using G = PerGroup<8>;
+    const int n = V.cnt->cur[S];
+    if (n > kForce4Max) return;
+    const auto one = [&](const Params& P, int i, bool valid) {
+        const float2 p = X.pos[i];
+        const float2 accB = wall_sum<A, G, S>(valid, P, V, p, cell_hash_s<0>(P, p));
+        if (valid && G::leader()) X.acc[i] = accB;
+    };
+    for_each_particle<G>(n, block, blocks, [&](int i, bool valid) {
+        if constexpr (B) one(V.table[sc[i]], i, valid);
+        else one(P0, i, valid);
+    });
+}
+
+template <class A, class G, int S>
+__device__ __forceinline__ float2 wall_term(bool valid, const Params& P, const StepView& V, const ScaleView& X, int i,
+                                            float2 p, int cell) {
+    if constexpr (G::kLanes == 8 || G::kLanes == 4) return X.acc[i];  // by_size's lists: wall_scale
+    else return wall_sum<A, G, S>(valid, P, V, p, cell);
+}
+
+// ---------------------------------------------------------------------------
 // Low-res density + Tait, computeParticleDensityPressure (WCSPHSolver.cu:1342-1424)
 // ---------------------------------------------------------------------------
 template <class A, class G>
@@ -455,12 +531,21 @@ template <bool B, class G, class A>
 __global__ void __launch_bounds__(256, B ? 6 : 8) k_density_low(Params P0, StepView V) {
     __shared__ int16_t s_nbr[G::kLanes > 1 ? 1 : kNbrRows * kNbrCols];
     int16_t* const nbr_col = s_nbr + (G::kLanes > 1 ? 0 : threadIdx.x);
+    const int blocks = gridDim.x - V.wallL - V.wallH;  // then the walls' blocks
+    const int block = static_cast<int>(blockIdx.x);
+    if (block >= blocks) {
+        if (block < blocks + V.wallL) wall_scale<B, A, 0>(P0, V, V.L, V.scL, block - blocks, V.wallL);
+        else wall_scale<B, A, 1>(P0, V, V.H, V.scH, block - blocks - V.wallL, V.wallH);
+        return;
+    }
     const bool cross = V.cnt->h_state0 != 0;
     // the split counts of the low-res force's tiles, zero before it
-    for (int t = tid(); t < (V.cnt->cur[0] + kSplitTile - 1) / kSplitTile; t += nthreads()) V.split_tile[t] = 0u;
+    for (int t = block * blockDim.x + threadIdx.x; t < (V.cnt->cur[0] + kSplitTile - 1) / kSplitTile;
+         t += blocks * blockDim.x)
+        V.split_tile[t] = 0u;
     by_size<G, false>(V.cnt->cur[0], [&](auto form, int n) {
         using F = decltype(form);
-        for_each_particle<F>(n, [&](int i, bool valid) {
+        for_each_particle<F>(n, block, blocks, [&](int i, bool valid) {
             if constexpr (B) {
                 const Params& P = V.table[V.scL[i]];
                 density_low_one<A, F>(P, V, i, valid, cross, nbr_col);
@@ -471,47 +556,12 @@ __global__ void __launch_bounds__(256, B ? 6 : 8) k_density_low(Params P0, StepV
     });
 }
 
-// Wall term of a force sum (updateAccCell 562-579 / updateAccCellComplementHigh
-// 867-884): every wall particle of the window's cells, in cell order.  Pairs with
-// sqrtf(x) > rad have q >= 2 and add exactly zero, so they are skipped.  S selects
-// the scale: 0 the low-res radius r, 1 the high-res radius rh.
-template <class A, class G, int S>
-__device__ __forceinline__ float2 wall_sum(bool on, const Params& P, const StepView& V, float2 p, int csx, int cex,
-                                           int csy, int cey, float Tle, float cB) {
-    float2 accB = make_float2(0.f, 0.f);
-    // A window of at most four cells a side from (csx, csy) lies within two cells of
-    // (mx, my); with no wall particle there the sum is empty.
-    if (cex - csx <= 3 && cey - csy <= 3) {
-        const int mx = min(csx + 1, P.dimL[0] - 1), my = min(csy + 1, P.dimL[1] - 1);
-        on = on && V.wnear[P.cbL + my * P.dimL[0] + mx];
-    }
-    if (!G::any(on)) return accB;
-    const int* woff = V.woff + P.cbL;
-    const float2* wpos = V.wpos + P.wb;
-    float2 pik = make_float2(0.f, 0.f);
-    float x = 0.0f;
-    G::window(
-        on, woff, P.dimL[0], csx, cex, csy, cey,
-        [&](int k) {
-            pik = sub(p, wpos[k]);
-            x = sq(pik);
-            return !(x > Tle);  // NaN passes: the reference's 0 * NaN offset propagates it
-        },
-        [&](int) { return A::template wall<S>(P, pik, x, cB); },
-        [](float2& a, float2 t) {
-            a.x += t.x;
-            a.y += t.y;
-        },
-        accB);
-    return accB;
-}
-
 // ---------------------------------------------------------------------------
 // Low-res force + advance + split test: computeParticleAcceleration
 // (WCSPHSolver.cu:1648-1865) with advance (1604-1646) fused; its predicted position
 // is the advanced position bit for bit.  The fluid and wall sums are independent
-// accumulators, so they are taken in two passes over the window.  The new position
-// also gives the entry's key for the next step's grid.  Returns the split flag.
+// accumulators.  The new position also gives the entry's
+// key for the next step's grid.  Returns the split flag.
 // ---------------------------------------------------------------------------
 template <class A, class G>
 __device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V, int i, bool valid, bool cross,
@@ -550,9 +600,8 @@ __device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V
             G::window(on, L.off + P.cbL, P.dimL[0], csx, cex, csy, cey, test, term, add_terms, fl);
         });
     }
-    grid_coord_s<0>(P, p.x, p.y, -P.r, csx, csy);
-    grid_coord_s<0>(P, p.x, p.y, P.r, cex, cey);
-    const float2 accB = wall_sum<A, G, 0>(valid, P, V, p, csx, cex, csy, cey, P.Tle_r, P.cBL);
+    const int cell = cell_hash_s<0>(P, p);
+    const float2 accB = wall_term<A, G, 0>(valid, P, V, L, i, p, cell);
     PairTerms fh{make_float2(0.f, 0.f), fl.t};  // (accH, accT): the sigma sum continues
     if (cross) {
         grid_coord_s<1>(P, p.x, p.y, -P.r, csx, csy);
@@ -606,18 +655,16 @@ __device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V
     if (valid && G::leader()) {
         L.acc[i] = acc;
         if (!isfinite(acc.x) || !isfinite(acc.y)) atomicOr(&V.cnt->err, kErrNumeric);
-        // a split parent's tether radius, 0.75 sqrt(m / (rho pi)) in double as the
-        // reference evaluates it (adjustPosition, WCSPHSolver.cu:1007-1022), once per
-        // parent here instead of once per child in the high-res force: FP64 is slow
-        // on this GPU.  min(dist, float(R)) == float(min(dist, R)) for a float dist
-        // (rounding is monotone), so the children's clamp is unchanged bit for bit.
-        if (s == 1u)
-            L.tr[i] = static_cast<float>(0.75 * sqrt(static_cast<double>(P.mL) / (static_cast<double>(dens) * kPi)));
+        // a split parent's tether radius (adjustPosition, WCSPHSolver.cu:1007-1022), once
+        // per parent here instead of once per child in the high-res force.  min(dist,
+        // float(R)) == float(min(dist, R)) for a float dist (rounding is monotone), so
+        // the children's clamp is unchanged bit for bit.
+        if (s == 1u) L.tr[i] = tether_radius(P, dens);
         // the cells of this step's grid that hold an entry in state 0 after the split
         // marks: the only low-res partners of a state-1 child in the high-res force.
         // The entry's cell is the one its key was made from (its position at the
         // start of the step, the same cell function).
-        if (ns == 0u) L.cflag[P.cbL + cell_hash_s<0>(P, L.pos[i])] = static_cast<uint8_t>(V.cnt->steps);
+        if (ns == 0u) L.cflag[P.cbL + cell] = static_cast<uint8_t>(V.cnt->steps);
         L.npos[i] = p;
         L.nvel[i] = v;
         L.nid[i] = L.id[i];
@@ -751,7 +798,7 @@ __device__ __forceinline__ void force_high_one(const Params& P, const StepView& 
             return A::template pair<kHCross>(P, pij, x, sub(v, vel_of(o)), qi, o.z, dens, o.w);
         },
         add_terms, fl);
-    const float2 accB = wall_sum<A, G, 1>(valid, P, V, p, csx, cex, csy, cey, P.Tle_rh, P.cBH);
+    const float2 accB = wall_term<A, G, 1>(valid, P, V, H, i, p, cell_hash_s<0>(P, p));
     float2 acc = fh.a, accL = fl.a;
     const float2 accT = fl.t;
     acc.x *= -P.mH;
@@ -846,7 +893,7 @@ void launch_gather_bg(int g, int blocks, int threads, cudaStream_t s, const Para
             k_density_high<B, G, A><<<blocks, threads, 0, s>>>(P, V);
             break;
         case 1:
-            k_density_low<B, G, A><<<blocks, threads, 0, s>>>(P, V);
+            k_density_low<B, G, A><<<blocks + V.wallL + V.wallH, threads, 0, s>>>(P, V);
             break;
         case 2:
             k_force_low<B, G, A><<<blocks, threads, 0, s>>>(P, V);

@@ -33,7 +33,7 @@ struct ScaleView {
     int16_t* nbr;
     uint8_t* nnbr;
     long long nbr_stride;  // entries per list column: the scale's capacity
-    float2* acc;
+    float2* acc;     // the accelerations; until the force, a short list's wall terms (wall_scale)
     const int* off;  // dense cell offsets [C+1]
     int32_t* map;    // slot id -> index in the cur arrays
     float2* npos;
@@ -61,6 +61,7 @@ struct StepView {
     float2* relax_pos;      // [capH] relaxation scratch
     float2* relax_vel;
     int nL;                 // low-res count (constant for a solver)
+    int wallL, wallH;       // the low-res density's last blocks: the two lists' wall terms
     // batches only: per-scene parameters and each sorted particle's scene
     const Params* table;
     const uint16_t* scL;
