@@ -1,5 +1,8 @@
 // grid.cu -- counting-sort grid build (see grid.cuh) and the tss_grid_build entry
 // point of the C ABI.
+#include <algorithm>
+#include <type_traits>
+
 #include <cuda_runtime.h>
 
 #include "../../include/tss.h"
@@ -25,12 +28,41 @@ int particle_blocks(int cap, int threads) {
     return b < 1 ? 1 : static_cast<int>(b);
 }
 
-__global__ void k_grid_keys(const float2* __restrict__ pos, const int* __restrict__ n_ptr, float ox, float oy,
-                            float cell, int dimx, int dimy, unsigned* __restrict__ count, int* __restrict__ key,
+// Entries taken per thread and trip: with four, their loads (and the atomics, whose
+// answers the ranks wait for) are in flight together; a list that does not fill the GPU
+// once is spread over more threads instead.
+constexpr int kUnroll = 4;
+constexpr int kUnrollMin = 150000;
+
+// f(std::integral_constant<int, U>) with the entries per trip for n
+template <class F>
+__device__ __forceinline__ void with_unroll(int n, F&& f) {
+    if (n < kUnrollMin) f(std::integral_constant<int, 1>{});
+    else f(std::integral_constant<int, kUnroll>{});
+}
+
+__global__ void k_grid_keys(const float2* __restrict__ pos, int* n_ptr, int n_set, float ox, float oy, float cell,
+                            int dimx, int dimy, unsigned* __restrict__ count, int* __restrict__ key,
                             int* __restrict__ rank, unsigned* __restrict__ tile_sum) {
-    const int n = *n_ptr;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        grid_key(count, key, rank, tile_sum, i, cell_hash(pos[i], ox, oy, cell, dimx, dimy));
+    let_next_start();
+    const int n = n_set >= 0 ? n_set : *n_ptr;
+    if (n_set >= 0 && blockIdx.x == 0 && threadIdx.x == 0) *n_ptr = n_set;
+    with_unroll(n, [&](auto unroll) {
+        constexpr int U = decltype(unroll)::value;
+        for (int base = blockIdx.x * blockDim.x * U; base < n; base += gridDim.x * blockDim.x * U) {
+            int c[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int i = base + u * blockDim.x + threadIdx.x;
+                c[u] = i < n ? cell_hash(pos[i], ox, oy, cell, dimx, dimy) : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int i = base + u * blockDim.x + threadIdx.x;
+                if (c[u] >= 0) grid_key(count, key, rank, tile_sum, i, c[u]);
+            }
+        }
+    });
 }
 
 // Tiles of kScanTile counts, strided over the blocks.  A tile's offset is the sum
@@ -40,6 +72,7 @@ __global__ void k_grid_keys(const float2* __restrict__ pos, const int* __restric
 // 16-byte groups that hold a non-zero count are written back).
 __global__ void __launch_bounds__(kScanThreads) k_grid_scan(GridBufs g) {
     let_next_start();
+    wait_for_previous();
     __shared__ unsigned s_warp[kScanThreads / 32];
     __shared__ unsigned s_red[kScanThreads / 32];
     const int C = g.used ? min(*g.used, g.ncells) : g.ncells;
@@ -160,38 +193,70 @@ __global__ void k_grid_scatter(const int* __restrict__ n_ptr, const int32_t* __r
         *g.nbig_snap = *g.nbig;
         *g.nbig = 0;  // empty for the next build's scan
     }
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int c = g.key[i];
-        if (c < 0) continue;  // dropped from the list
-        if (c >= g.ncells) {
-            atomicOr(err, kErrGridIndex);
-            continue;
+    with_unroll(n, [&](auto unroll) {
+        constexpr int U = decltype(unroll)::value;
+        for (int base = blockIdx.x * blockDim.x * U; base < n; base += gridDim.x * blockDim.x * U) {
+            int c[U], r[U], d[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int i = base + u * blockDim.x + threadIdx.x;
+                c[u] = i < n ? g.key[i] : -1;  // negative: dropped from the list
+                r[u] = i < n ? g.rank[i] : 0;
+                d[u] = i < n ? id[i] : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int i = base + u * blockDim.x + threadIdx.x;
+                if (c[u] < 0) continue;
+                if (c[u] >= g.ncells) {
+                    atomicOr(err, kErrGridIndex);
+                    continue;
+                }
+                const int s = g.off[c[u]], k = g.off[c[u] + 1] - s;
+                const int dst = s + r[u];
+                if (dst < 0 || dst >= total) {
+                    atomicOr(err, kErrGridIndex);
+                    continue;
+                }
+                g.perm[dst] = make_int2(i, d[u]);
+                g.place[dst] = k <= kBigCell ? (k << 8) | (r[u] & 255) : -1;
+            }
         }
-        const int dst = g.off[c] + g.rank[i];
-        if (dst < 0 || dst >= total) {
-            atomicOr(err, kErrGridIndex);
-            continue;
-        }
-        g.perm[dst] = make_int2(i, id[i]);
-    }
+    });
 }
 
 namespace {
 
-// Gathers list entry src's state into sorted position dst.
-__device__ __forceinline__ void reorder_move(const ReorderArgs& a, int src, int dst, int id, unsigned* err) {
-    if (a.dst_pos) a.dst_pos[dst] = a.src_pos[src];
-    if (a.src_vel) *reinterpret_cast<float2*>(&a.dst_vq[dst]) = a.src_vel[src];
+// A list entry's state, on its way to its sorted place.
+struct Moved {
+    float2 pos, vel;
+    uint8_t st;
+    float dens, pres;
+};
+__device__ __forceinline__ Moved reorder_load(const ReorderArgs& a, int src) {
+    Moved m{};
+    if (a.dst_pos) m.pos = a.src_pos[src];
+    if (a.src_vel) m.vel = a.src_vel[src];
+    if (a.src_st) m.st = a.src_st[src];
+    if (a.src_dens) {
+        m.dens = a.src_dens[src];
+        m.pres = a.src_pres[src];
+    }
+    return m;
+}
+__device__ __forceinline__ void reorder_store(const ReorderArgs& a, const Moved& m, int src, int dst, int id,
+                                              unsigned* err) {
+    if (a.dst_pos) a.dst_pos[dst] = m.pos;
+    if (a.src_vel) *reinterpret_cast<float2*>(&a.dst_vq[dst]) = m.vel;
     if (a.src_st) {
-        uint8_t st = a.src_st[src];
-        a.dst_st[dst] = st;
-        if (a.h_state0 && (st & 1u) == 0u) *a.h_state0 = 1;
-        if (a.deleted && st >= 2u) *a.deleted = 1;
+        a.dst_st[dst] = m.st;
+        if (a.h_state0 && (m.st & 1u) == 0u) *a.h_state0 = 1;
+        if (a.deleted && m.st >= 2u) *a.deleted = 1;
     }
     if (a.dst_id) a.dst_id[dst] = id;
     if (a.src_dens) {
-        a.dst_dens[dst] = a.src_dens[src];
-        a.dst_pres[dst] = a.src_pres[src];
+        a.dst_dens[dst] = m.dens;
+        a.dst_pres[dst] = m.pres;
     }
     if (a.dst_order) a.dst_order[dst] = src;
     if (a.dst_sc) a.dst_sc[dst] = a.page_scene[(id >> a.id_shift) >> a.page_shift];
@@ -310,26 +375,19 @@ __global__ void __launch_bounds__(kReorderThreads) k_grid_reorder(int* n_ptr, in
     const int tiles = ((g.used ? min(*g.used, g.ncells) : g.ncells) + kScanTile - 1) / kScanTile;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < tiles; t += gridDim.x * blockDim.x) g.tile_sum[t] = 0u;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        int2 pe = g.perm[k];
+        const int2 pe = g.perm[k];
+        const int w = g.place[k];
         const int src = pe.x, id = pe.y;
-        if (src < 0 || src >= cap) {
+        if (w < 0) continue;  // a big cell's: placed below
+        const int s = k - (w & 255), e = s + (w >> 8);
+        if (src < 0 || src >= cap || s < 0 || e > n || k >= e) {
             atomicOr(err, kErrGridIndex);
             continue;
         }
-        const int c = g.key[src];
-        if (c < 0 || c >= g.ncells) {
-            atomicOr(err, kErrGridIndex);
-            continue;
-        }
-        const int s = g.off[c], e = g.off[c + 1];
-        if (s < 0 || e > n || s > k || k >= e) {
-            atomicOr(err, kErrGridIndex);
-            continue;
-        }
-        if (e - s > kBigCell) continue;  // placed below, with its cell
+        const Moved m = reorder_load(a, src);  // in flight while the cell's ids are counted
         int r = 0;
         for (int j = s; j < e; ++j) r += g.perm[j].y < id;
-        reorder_move(a, src, s + r, id, err);
+        reorder_store(a, m, src, s + r, id, err);
     }
     const int nb = min(*g.nbig_snap, g.big_cap);
     for (int b = blockIdx.x; b < nb; b += gridDim.x) {
@@ -344,7 +402,7 @@ __global__ void __launch_bounds__(kReorderThreads) k_grid_reorder(int* n_ptr, in
             continue;
         }
         const int k = e - s;
-        const int* sorted = block_sort_ids(g.perm + s, k, g.rank + s, g.sortbuf + s);
+        const int* sorted = block_sort_ids(g.perm + s, k, g.rank + s, g.key + s);
         __syncthreads();
         for (int j = threadIdx.x; j < k; j += blockDim.x) {
             const int2 pe = g.perm[s + j];
@@ -353,7 +411,7 @@ __global__ void __launch_bounds__(kReorderThreads) k_grid_reorder(int* n_ptr, in
                 atomicOr(err, kErrGridIndex);
                 continue;
             }
-            reorder_move(a, src, s + lower_rank(sorted, k, id), id, err);
+            reorder_store(a, reorder_load(a, src), src, s + lower_rank(sorted, k, id), id, err);
         }
         __syncthreads();  // the buffers are reused by the block's next cell
     }
@@ -371,6 +429,13 @@ size_t grid_bufs_bytes(int cap, int ncells, bool own_off, bool own_sort) {
            al(sizeof(int) * big_cap) + 256;
 }
 
+// What must be zero before the key pass comes first: counts, tile sums, counters.
+size_t grid_clear_bytes(int ncells) {
+    auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
+    const int ntiles = std::max((ncells + kScanTile - 1) / kScanTile, 1);
+    return al(sizeof(unsigned) * (size_t)ncells) + al(sizeof(unsigned) * (size_t)ntiles) + 256;
+}
+
 GridBufs grid_bufs_carve(void* base, int cap, int ncells, bool own_off, bool own_sort) {
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
     char* p = static_cast<char*>(base);
@@ -380,6 +445,13 @@ GridBufs grid_bufs_carve(void* base, int cap, int ncells, bool own_off, bool own
     if (g.ntiles < 1) g.ntiles = 1;
     g.count = reinterpret_cast<unsigned*>(p);
     p += al(sizeof(unsigned) * (size_t)ncells);
+    g.tile_sum = reinterpret_cast<unsigned*>(p);
+    p += al(sizeof(unsigned) * (size_t)g.ntiles);
+    g.used = nullptr;
+    g.total = reinterpret_cast<int*>(p);  // 256 bytes: total, nbig, nbig_snap
+    g.nbig = g.total + 1;
+    g.nbig_snap = g.total + 2;
+    p += 256;
     g.off = nullptr;
     if (own_off) {
         g.off = reinterpret_cast<int*>(p);
@@ -389,35 +461,28 @@ GridBufs grid_bufs_carve(void* base, int cap, int ncells, bool own_off, bool own
     p += al(sizeof(int) * (size_t)cap);
     g.rank = reinterpret_cast<int*>(p);
     p += al(sizeof(int) * (size_t)cap);
-    g.sortbuf = nullptr;
+    g.place = nullptr;
     g.perm = nullptr;
     if (own_sort) {
-        g.sortbuf = reinterpret_cast<int*>(p);
+        g.place = reinterpret_cast<int*>(p);
         p += al(sizeof(int) * (size_t)cap);
         g.perm = reinterpret_cast<int2*>(p);
         p += al(sizeof(int2) * (size_t)cap);
     }
-    g.tile_sum = reinterpret_cast<unsigned*>(p);
-    p += al(sizeof(unsigned) * (size_t)g.ntiles);
     g.big_cap = cap / (kBigCell + 1) + 1;
     g.big = reinterpret_cast<int*>(p);
-    p += al(sizeof(int) * static_cast<size_t>(g.big_cap));
-    g.used = nullptr;
-    g.total = reinterpret_cast<int*>(p);  // the last 256 bytes: total, nbig, nbig_snap
-    g.nbig = g.total + 1;
-    g.nbig_snap = g.total + 2;
     return g;
 }
 
 void grid_lend_sort(GridBufs& g, void* mem, int cap) {
     g.perm = static_cast<int2*>(mem);
-    g.sortbuf = reinterpret_cast<int*>(g.perm + cap);
+    g.place = reinterpret_cast<int*>(g.perm + cap);
 }
 
-cudaError_t grid_keys_enqueue(const float2* pos, const int* n_ptr, int cap, float ox, float oy, float cell, int dimx,
-                              int dimy, GridBufs g, cudaStream_t stream) {
+cudaError_t grid_keys_enqueue(const float2* pos, int* n_ptr, int cap, float ox, float oy, float cell, int dimx,
+                              int dimy, GridBufs g, cudaStream_t stream, int n_set) {
     const int T = 256;
-    k_grid_keys<<<particle_blocks(cap, T), T, 0, stream>>>(pos, n_ptr, ox, oy, cell, dimx, dimy, g.count, g.key,
+    k_grid_keys<<<particle_blocks(cap, T), T, 0, stream>>>(pos, n_ptr, n_set, ox, oy, cell, dimx, dimy, g.count, g.key,
                                                            g.rank, g.tile_sum);
     return cudaGetLastError();
 }
@@ -425,11 +490,11 @@ cudaError_t grid_keys_enqueue(const float2* pos, const int* n_ptr, int cap, floa
 cudaError_t grid_sort_enqueue(const int32_t* id, int* n_ptr, int cap, GridBufs g, ReorderArgs a,
                               unsigned* err, cudaStream_t stream) {
     const int T = 256;
-    const int pb = particle_blocks(cap, T);
     const int sb = g.ntiles < 8 * sm_count() ? g.ntiles : 8 * sm_count();
-    k_grid_scan<<<sb, kScanThreads, 0, stream>>>(g);
-    cudaError_t e = launch_after(k_grid_scatter, pb, T, stream, n_ptr, id, g, err);
-    if (e == cudaSuccess) e = launch_after(k_grid_reorder, pb, kReorderThreads, stream, n_ptr, cap, g, a, err);
+    cudaError_t e = launch_after(k_grid_scan, sb, kScanThreads, stream, g);
+    if (e == cudaSuccess) e = launch_after(k_grid_scatter, particle_blocks(cap, T), T, stream, n_ptr, id, g, err);
+    if (e == cudaSuccess)
+        e = launch_after(k_grid_reorder, particle_blocks(cap, kReorderThreads), kReorderThreads, stream, n_ptr, cap, g, a, err);
     return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
@@ -484,12 +549,14 @@ extern "C" tss_status tss_grid_build(const float* d_pos, const int32_t* d_id, in
     unsigned* err = reinterpret_cast<unsigned*>(n_dev + 2);
     tss::GridBufs g = tss::grid_bufs_carve(w + 256, cap, cells, false);
     g.off = d_cell_off;  // write the offsets straight into the caller's table
-    if (cudaMemsetAsync(w, 0, 256, st) != cudaSuccess) return TSS_CUDA_ERROR;
-    tss::k_set_int<<<1, 1, 0, st>>>(n_dev, n);
+    // one clear (count and error word, and the grid's counts behind them), then the kernels
+    cudaError_t e = cudaMemsetAsync(w, 0, 256 + tss::grid_clear_bytes(cells), st);
     tss::ReorderArgs a{};  // only the order is gathered
     a.src_pos = reinterpret_cast<const float2*>(d_pos);
     a.dst_order = d_order;
-    cudaError_t e = tss::grid_build_enqueue(reinterpret_cast<const float2*>(d_pos), d_id, n_dev, cap, origin_x, origin_y,
-                                            cell_size, dimx, dimy, g, a, err, st);
+    if (e == cudaSuccess)
+        e = tss::grid_keys_enqueue(reinterpret_cast<const float2*>(d_pos), n_dev, cap, origin_x, origin_y, cell_size,
+                                   dimx, dimy, g, st, n);
+    if (e == cudaSuccess) e = tss::grid_sort_enqueue(d_id, n_dev, cap, g, a, err, st);
     return e == cudaSuccess ? TSS_OK : TSS_CUDA_ERROR;
 }

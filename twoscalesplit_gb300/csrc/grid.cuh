@@ -15,8 +15,10 @@
 //   k_grid_scan     off = exclusive_scan(count) over the cells in use: each tile
 //                   adds the sums of the tiles before it; count is zeroed for the
 //                   next build; off[used] = total = the number of keyed entries
-//   k_grid_scatter  perm[off[key[i]] + rank[i]] = (i, id[i]); entries whose key is
-//                   negative (removed since their key pass) are dropped
+//   k_grid_scatter  perm[off[key[i]] + rank[i]] = (i, id[i]), with the cell's size and
+//                   the slot's rank in it beside it (place), so that the reorder needs
+//                   no way back to its cell; entries whose key is negative (removed
+//                   since their key pass) are dropped
 //   k_grid_reorder  each sorted slot finds its final place in its cell, ascending
 //                   id, and gathers the particle's state there (SoA reorder); the
 //                   list count becomes the sorted count.  In a cell of at most
@@ -32,6 +34,13 @@
 
 namespace tss {
 
+// The scatter and the reorder wait for chains of dependent loads (a fifth of the copy
+// rate at 1.0M entries).  With four of the scatter's entries in flight per thread, and
+// the reorder going from the permutation to the cell's ids without the key and the
+// offsets between (its state loads in flight meanwhile), a build of 1.0M entries in the
+// step took 37 -> 33 us; the step of 1.0M + 1.0M particles 364 -> 359 us, of 5,000
+// (graphs of eight) 31.8 -> 30.5 us.
+//
 // A scan tile of 2048 cells: the grids have about as many cells as particles, so
 // the scan is latency-bound; 2048-cell tiles give the 1M-particle scene's 3.1M-cell
 // high-res grid 1526 tiles (8 blocks per SM, one or two tiles each) and scanned it
@@ -60,7 +69,7 @@ struct GridBufs {
     int big_cap;            // cap / (kBigCell + 1) + 1
     int* nbig;              // device int: cells appended by the scan (the scatter resets it)
     int* nbig_snap;         // device int: ... as the scatter found it, for the reorder
-    int* sortbuf;           // [cap] ids of the big cells while they are sorted (with rank)
+    int* place;             // [cap] per sorted slot, its cell's entries << 8 | its rank; -1: a big cell's
 };
 
 // What the reorder moves: list-order arrays (src) into sorted-order arrays (dst).
@@ -89,8 +98,8 @@ struct ReorderArgs {
     int* deleted;              // may be null: set to 1 if some entry has state >= 2
 };
 
-__global__ void k_grid_keys(const float2* __restrict__ pos, const int* __restrict__ n_ptr, float ox, float oy,
-                            float cell, int dimx, int dimy, unsigned* __restrict__ count, int* __restrict__ key,
+__global__ void k_grid_keys(const float2* __restrict__ pos, int* n_ptr, int n_set, float ox, float oy, float cell,
+                            int dimx, int dimy, unsigned* __restrict__ count, int* __restrict__ key,
                             int* __restrict__ rank, unsigned* __restrict__ tile_sum);
 __global__ void k_grid_scan(GridBufs g);
 __global__ void k_grid_scatter(const int* __restrict__ n_ptr, const int32_t* __restrict__ id, GridBufs g,
@@ -135,8 +144,9 @@ cudaError_t grid_build_enqueue(const float2* pos, const int32_t* id, int* n_ptr,
 // (scan, scatter, reorder, which clears the tile sums for the next key pass).  The
 // solver's step runs the key pass inside its force kernels (grid_key below) and
 // only the rest here.
-cudaError_t grid_keys_enqueue(const float2* pos, const int* n_ptr, int cap, float ox, float oy, float cell, int dimx,
-                              int dimy, GridBufs g, cudaStream_t stream);
+// n_set >= 0: the list's length, which the key pass also writes to *n_ptr.
+cudaError_t grid_keys_enqueue(const float2* pos, int* n_ptr, int cap, float ox, float oy, float cell, int dimx,
+                              int dimy, GridBufs g, cudaStream_t stream, int n_set = -1);
 cudaError_t grid_sort_enqueue(const int32_t* id, int* n_ptr, int cap, GridBufs g, ReorderArgs a,
                               unsigned* err, cudaStream_t stream);
 
@@ -154,10 +164,12 @@ __device__ __forceinline__ void grid_key(unsigned* __restrict__ count, int* __re
 
 // Device bytes of a grid's buffers for `cap` entries and `ncells` cells.  own_off =
 // false leaves out the offset table (the caller then sets g.off to its own).
-// own_sort = false leaves out perm and sortbuf, which only live within a build: the
+// own_sort = false leaves out perm and place, which only live within a build: the
 // caller lends the build grid_sort_bytes(cap) that are dead then (grid_lend_sort).
 size_t grid_bufs_bytes(int cap, int ncells, bool own_off = true, bool own_sort = true);
 GridBufs grid_bufs_carve(void* base, int cap, int ncells, bool own_off = true, bool own_sort = true);
+// The bytes at their start that a key pass needs zero (counts, tile sums, counters).
+size_t grid_clear_bytes(int ncells);
 constexpr size_t grid_sort_bytes(size_t cap) { return cap * (sizeof(int2) + sizeof(int)); }
 void grid_lend_sort(GridBufs& g, void* mem, int cap);
 

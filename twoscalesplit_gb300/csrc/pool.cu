@@ -433,6 +433,7 @@ tss_status admit(tss_solver* s, const SceneIn& in, cudaStream_t st, int* scene_i
         gv.key = s->gW.key + wb;
         gv.rank = s->gW.rank + wb;
         gv.perm = s->gW.perm + wb;
+        gv.place = s->gW.place + wb;
         gv.used = nullptr;
         ReorderArgs a{};
         a.src_pos = s->wraw + wb;
