@@ -65,6 +65,41 @@ __global__ void k_grid_keys(const float2* __restrict__ pos, int* n_ptr, int n_se
     });
 }
 
+// The particles of each tile of kScanTile cells, from the finished counts (a key pass of
+// many entries does not add them up itself: grid_keys_enqueue).
+__global__ void __launch_bounds__(kScanThreads) k_grid_tiles(GridBufs g) {
+    __shared__ unsigned s_sum[kScanThreads / 32];
+    let_next_start();
+    wait_for_previous();
+    const int C = g.used ? min(*g.used, g.ncells) : g.ncells;
+    const int ntiles = (C + kScanTile - 1) / kScanTile;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int base = tile * kScanTile + threadIdx.x * kScanItems;
+        unsigned sum = 0;
+        if (base + kScanItems <= C) {
+            const uint4* p = reinterpret_cast<const uint4*>(g.count + base);
+#pragma unroll
+            for (int q = 0; q < kScanItems / 4; ++q) {
+                const uint4 v = p[q];
+                sum += v.x + v.y + v.z + v.w;
+            }
+        } else {
+            for (int k = 0; k < kScanItems; ++k)
+                if (base + k < C) sum += g.count[base + k];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = sum;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            unsigned t = 0;
+            for (int w = 0; w < kScanThreads / 32; ++w) t += s_sum[w];
+            g.tile_sum[tile] = t;
+        }
+        __syncthreads();
+    }
+}
+
 // Tiles of kScanTile counts, strided over the blocks.  A tile's offset is the sum
 // of the tile sums before it (read from L2), so tiles are independent and nothing
 // waits on another block.  Only the cells in use are scanned (a pool's grids are
@@ -482,9 +517,18 @@ void grid_lend_sort(GridBufs& g, void* mem, int cap) {
 cudaError_t grid_keys_enqueue(const float2* pos, int* n_ptr, int cap, float ox, float oy, float cell, int dimx,
                               int dimy, GridBufs g, cudaStream_t stream, int n_set) {
     const int T = 256;
+    // A key pass alone is bound by its atomics, above all by those of neighbouring warps
+    // on the same tile sums: without them 1.3M points take 13 us instead of 29, and the
+    // sums are read off the counts in a kernel of 4 us (the whole build 59 -> 45 us; at
+    // 200,000 points 23.5 -> 21 us, at 20,000 no faster).  The steps' key passes hide them
+    // in the force kernels: there, the extra kernel costs 3 us of 360.
+    const bool apart = cap >= kUnrollMin;
     k_grid_keys<<<particle_blocks(cap, T), T, 0, stream>>>(pos, n_ptr, n_set, ox, oy, cell, dimx, dimy, g.count, g.key,
-                                                           g.rank, g.tile_sum);
-    return cudaGetLastError();
+                                                           g.rank, apart ? nullptr : g.tile_sum);
+    cudaError_t e = cudaGetLastError();
+    if (apart && e == cudaSuccess)
+        e = launch_after(k_grid_tiles, g.ntiles < 8 * sm_count() ? g.ntiles : 8 * sm_count(), kScanThreads, stream, g);
+    return e;
 }
 
 cudaError_t grid_sort_enqueue(const int32_t* id, int* n_ptr, int cap, GridBufs g, ReorderArgs a,

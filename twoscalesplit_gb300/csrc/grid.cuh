@@ -11,7 +11,8 @@
 //
 //   k_grid_keys     key[i] = cell(pos[i]); rank[i] = atomicAdd(&count[cell], 1);
 //                   per tile of kScanTile cells, the number of particles
-//                   (warp-aggregated atomics), so the scan needs no look-back
+//                   (warp-aggregated atomics, or k_grid_tiles from the counts), so the
+//                   scan needs no look-back
 //   k_grid_scan     off = exclusive_scan(count) over the cells in use: each tile
 //                   adds the sums of the tiles before it; count is zeroed for the
 //                   next build; off[used] = total = the number of keyed entries
@@ -151,12 +152,14 @@ cudaError_t grid_sort_enqueue(const int32_t* id, int* n_ptr, int cap, GridBufs g
                               unsigned* err, cudaStream_t stream);
 
 // The key of list entry i for the next build: its cell, its rank among the cell's
-// entries (atomic order; the reorder fixes the order by id) and the tile sum.
+// entries (atomic order; the reorder fixes the order by id) and the tile sum (unless
+// tile_sum is null).
 // Lanes of a warp that hit the same tile add once.
 __device__ __forceinline__ void grid_key(unsigned* __restrict__ count, int* __restrict__ key, int* __restrict__ rank,
                                          unsigned* __restrict__ tile_sum, int i, int c) {
     key[i] = c;
     rank[i] = static_cast<int>(atomicAdd(&count[c], 1u));
+    if (!tile_sum) return;
     const unsigned t = static_cast<unsigned>(c) / kScanTile;
     const unsigned peers = __match_any_sync(__activemask(), t);
     if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&tile_sum[t], static_cast<unsigned>(__popc(peers)));
