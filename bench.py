@@ -642,7 +642,7 @@ def run_ours(args):
         "e2e": {"value": parts_all / ex["e2e_s"], "unit": UNIT, "h2d_bytes_per_step": ex["h2d"] / K,
                 "d2h_bytes_per_step": ex["d2h"] / K},
         # kernels per step: 2 grid sorts x 3 (scan, scatter, reorder), 4 gathers, split
-        # compaction, finish (+ 3 per relaxation sub-step); the 3 memset nodes are not counted
+        # compaction, finish (+ 3 per relaxation sub-step); no memset nodes
         "gpu_launches": K * (12 + 3 * cfg.relax_iters),
         "clocks": ex["clk"],
         "wall_s_timed": ex["wall"],

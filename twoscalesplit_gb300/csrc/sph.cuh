@@ -24,8 +24,8 @@ struct ScaleView {
     // (mod 256) when the cell holds an entry in state 0 after the split marks.  Any
     // other value only makes the high-res force walk a row it could skip.
     uint8_t* cflag;
-    // Neighbour lists the density pass records for the force pass of the same scale
-    // (one particle per thread): entry c of sorted particle i is
+    // Neighbour lists the density pass records for the force pass of the same scale:
+    // entry c of sorted particle i is
     // nbr[c * nbr_stride + i] = j - i for its c-th same-scale neighbour within the
     // density's support (itself left out), in window order; nnbr[i] is their count,
     // kNbrOverflow when there are more than kMaxNbr or an offset does not fit 16
