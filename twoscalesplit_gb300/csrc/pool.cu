@@ -670,7 +670,7 @@ tss_status tss_batch_create(int n_scenes, const tss_scene_desc* scenes, int cap_
     tss_solver* s = nullptr;
     tss_status st = create_pool(c, false, &s);
     if (st != TSS_OK) return st;
-    s->blocksL = (s->nL + 255) / 256;  // the low-res list is full: one block per 256 particles
+    s->blocksL = (s->nL + 255) / 256;  // the low-res list starts full but for its pages' rounding: one block per 256 slots
     s->low_full = true;
     if ((st = s->apply_launch(default_launch())) != TSS_OK) {
         delete s;

@@ -148,7 +148,9 @@ cudaError_t tss_solver::enqueue_step(cudaStream_t s) {
         const long long t = launch.threads[1], want = (8LL * std::min(cap, kForce4Max) + t - 1) / t;
         return static_cast<int>(std::min(want, 4LL * sm_count() * 256 / t));
     };
-    V.wallL = low_full && nL > kForce4Max ? 0 : wall_blocks(nL);  // a full list stays as long as it is
+    // none for a list that the kernels cannot find short: a single scene's count never
+    // changes, while a batch or pool has a capacity in whole pages and scenes that leave
+    V.wallL = !batched && nL > kForce4Max ? 0 : wall_blocks(nL);
     V.wallH = wall_blocks(capH);
     if (branch && (e = fork()) != cudaSuccess) return e;
     // the shorter density goes to the GPU before the longer: 278 us a step at 1.0M + 1.0M

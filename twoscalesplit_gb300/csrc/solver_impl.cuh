@@ -125,7 +125,9 @@ struct tss_solver {
     cudaGraph_t graph[kBuckets] = {};
     cudaGraphExec_t exec[kBuckets] = {};
     int blocksL = 1, blocksH = 1;           // the non-gather particle kernels
-    bool low_full = true;                   // the low-res list is always full (single scenes, batches)
+    // the low-res list is sized for its particles: full in a single scene, in a batch full
+    // up to its pages' rounding until a scene is retired (pools: false)
+    bool low_full = true;
     tss_launch launch{};                    // the gathers' launch shape
     int arith = TSS_ARITH_EXACT;            // the gathers' arithmetic (tss_solver_set_arith)
     int gather_grid[TSS_NUM_GATHERS] = {};  // blocks of each gather for that shape
