@@ -148,7 +148,11 @@ __device__ __forceinline__ int nbr_search(const int* off, int dimx, int csx, int
 }
 
 // Phase two: adds the terms of the n entries in the column to `sum`, in order, and
-// writes the entries other than the particle itself to its neighbour list.
+// writes the entries other than the particle itself to its neighbour list.  The column
+// holds one entry more than the list; the particle itself is not always among them, for
+// the relaxation moves children after the grid is built.  Only the entry past the last
+// pair can be one too many (a bound tested at every entry put 1 % on a step of 1.0M +
+// 1.0M particles).
 template <class A>
 __device__ __forceinline__ void nbr_density(const Params& P, const ScaleView& S, int i, float2 p, int n,
                                             const int16_t* col, float& sum) {
@@ -170,11 +174,16 @@ __device__ __forceinline__ void nbr_density(const Params& P, const ScaleView& S,
         entry(d0, x0);
         entry(d1, x1);
     }
+    static_assert(kMaxNbr % 2 == 0, "entry kMaxNbr is not half of a pair");
     if (c < n) {
         const int d0 = col[c * kNbrCols];
-        entry(d0, sq(sub(p, S.pos[i + d0])));
+        sum += A::density(P, sq(sub(p, S.pos[i + d0])));
+        if (d0 != 0) {
+            if (m < kMaxNbr) *dst = static_cast<int16_t>(d0);
+            ++m;
+        }
     }
-    S.nnbr[i] = static_cast<uint8_t>(m);
+    S.nnbr[i] = m <= kMaxNbr ? static_cast<uint8_t>(m) : kNbrOverflow;
 }
 
 // A same-scale neighbour's state as the force pass reads it.
