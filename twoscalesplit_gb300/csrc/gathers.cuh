@@ -99,7 +99,8 @@ using namespace gather_detail;
 // accept different candidates of the ~34 in their windows, so a walk that evaluates
 // a pair as soon as its test passes runs the pair arithmetic for nearly every
 // candidate with a third of the lanes active; here it runs once per list entry with
-// almost all of them (the lists are 10-14 long).  A dam break of 1.0M low-res and
+// almost all of them (the lists are 10-14 long).  A window of more particles than a list
+// holds is taken column by column (nbr_crowd).  A dam break of 1.0M low-res and
 // 1.0M high-res particles, exact / tolerance arithmetic, against a walk that
 // evaluated at once: low-res density 96 -> 61 / 73 -> 51 us, high-res density 117 ->
 // 86 / 92 -> 67 us (with the longer lists, kMaxNbr); a 5,000-particle scene 16 -> 13
@@ -109,31 +110,37 @@ constexpr int kNbrCols = 256;          // the gathers' largest block
 constexpr int kNbrRows = kMaxNbr + 5;  // the particle itself, and one trip of four past a full list
 
 // Phase one: the candidates k of the window with key(k) <= T (a NaN key fails), in
-// window order, as k - i in the column.  Returns their number, or -1 when there are
-// more than the list holds or an offset does not fit 16 bits.
+// window order, as k - i in the column.  Returns their number; kNbrFar when an offset
+// does not fit 16 bits; or, when there are more than the list holds, minus the number
+// found before the search stopped, at candidate k of row cy.
+constexpr int kNbrFar = -0x10000;
+
 template <class Key>
-__device__ __forceinline__ int nbr_search(const int* off, int dimx, int csx, int cex, int csy, int cey, int i, float T,
-                                          int16_t* col, Key&& key) {
+__device__ __forceinline__ int nbr_search(const int* off, int dimx, int csx, int cex, int& cy, int cey, int& k, int i,
+                                          float T, int16_t* col, Key&& key) {
     int16_t* c = col;
     int16_t* const full = col + (kMaxNbr + 1) * kNbrCols;
-    const auto put = [&](int k, float x) {
+    const auto put = [&](int j, float x) {
         if (x <= T) {
-            *c = static_cast<int16_t>(k - i);
+            *c = static_cast<int16_t>(j - i);
             c += kNbrCols;
         }
     };
-    for (int cy = csy; cy <= cey; ++cy) {
+    for (; cy <= cey; ++cy) {
         const int row = cy * dimx;
-        int k = off[row + csx];
+        k = off[row + csx];
         const int b = off[row + cex + 1];
-        if (k - i < -32768 || b - i > 32768) return -1;
+        if (k - i < -32768 || b - i > 32768) return kNbrFar;
         for (; k + 3 < b; k += 4) {
             const float x0 = key(k), x1 = key(k + 1), x2 = key(k + 2), x3 = key(k + 3);
             put(k, x0);
             put(k + 1, x1);
             put(k + 2, x2);
             put(k + 3, x3);
-            if (c > full) return -1;
+            if (c > full) {
+                k += 4;
+                return -(static_cast<int>(c - col) / kNbrCols);
+            }
         }
         if (k + 1 < b) {
             const float x0 = key(k), x1 = key(k + 1);
@@ -141,10 +148,62 @@ __device__ __forceinline__ int nbr_search(const int* off, int dimx, int csx, int
             put(k + 1, x1);
             k += 2;
         }
-        if (k < b) put(k, key(k));
-        if (c > full) return -1;
+        if (k < b) {
+            put(k, key(k));
+            ++k;
+        }
+        if (c > full) return -(static_cast<int>(c - col) / kNbrCols);
     }
     return static_cast<int>(c - col) / kNbrCols;
+}
+
+// The rest of a window that holds more than a list: adds the terms of the n entries in
+// the column, searches on from candidate k of row cy until the column is full again, and
+// so on, so that a warp's lanes evaluate their pairs together here too.  Returns false
+// when it comes to a row that does not fit 16 bits.  With a support of 3 lattice spacings
+// (28 neighbours, 81 candidates) the exact low-res density of 700,000 particles takes 123
+// us, of 4 spacings (50, 144) 156 us; a walk that evaluates at once took 125 and 203 us,
+// and after a search that gave up 320 and 430 us.
+template <class A, class Key>
+__device__ __forceinline__ bool nbr_crowd(const Params& P, const ScaleView& S, const int* off, int dimx, int csx,
+                                          int cex, int cy, int cey, int k, int i, float2 p, float T, int16_t* col,
+                                          int n, float& sum, Key&& key) {
+    int16_t* const full = col + (kMaxNbr + 1) * kNbrCols;
+    int16_t* c = col + n * kNbrCols;
+    int b = off[cy * dimx + cex + 1];
+    bool fit = true, done = false;
+    while (!done) {
+        for (const int16_t* q = col; q < c; q += kNbrCols) sum += A::density(P, sq(sub(p, S.pos[i + *q])));
+        c = col;
+        done = !fit || cy > cey;
+        while (fit && cy <= cey && c <= full) {
+            if (k + 3 < b) {
+                const float x0 = key(k), x1 = key(k + 1), x2 = key(k + 2), x3 = key(k + 3);
+                const auto put = [&](int j, float x) {
+                    if (x <= T) {
+                        *c = static_cast<int16_t>(j - i);
+                        c += kNbrCols;
+                    }
+                };
+                put(k, x0);
+                put(k + 1, x1);
+                put(k + 2, x2);
+                put(k + 3, x3);
+                k += 4;
+            } else if (k < b) {
+                if (key(k) <= T) {
+                    *c = static_cast<int16_t>(k - i);
+                    c += kNbrCols;
+                }
+                ++k;
+            } else if (++cy <= cey) {
+                k = off[cy * dimx + csx];
+                b = off[cy * dimx + cex + 1];
+                fit = k - i >= -32768 && b - i <= 32768;
+            }
+        }
+    }
+    return fit;
 }
 
 // Phase two: adds the terms of the n entries in the column to `sum`, in order, and
@@ -289,12 +348,20 @@ __device__ __forceinline__ void same_scale_density(bool on, const Params& P, con
         }
         if (on && G::leader()) S.nnbr[i] = n <= kMaxNbr && fit ? static_cast<uint8_t>(n) : kNbrOverflow;
     } else {
-        const int n = nbr_search(off, dimx, csx, cex, csy, cey, i, T, nbr_col, key);
+        int cy = csy, at = 0;
+        // the lanes leave the search at different candidates; without a barrier here those
+        // with too many went on alone (123 -> 195 us in the example at nbr_crowd)
+        const unsigned together = __activemask();
+        const int n = nbr_search(off, dimx, csx, cex, cy, cey, at, i, T, nbr_col, key);
+        __syncwarp(together);
         if (n >= 0) {
             nbr_density<A>(P, S, i, p, n, nbr_col, sum);
-        } else {
-            S.nnbr[i] = kNbrOverflow;
+            return;
+        }
+        S.nnbr[i] = kNbrOverflow;
+        if (n == kNbrFar || !nbr_crowd<A>(P, S, off, dimx, csx, cex, cy, cey, at, i, p, T, nbr_col, -n, sum, key)) {
             float x = 0.0f;
+            sum = 0.0f;
             G::window(
                 true, off, dimx, csx, cex, csy, cey,
                 [&](int k) {
