@@ -42,6 +42,6 @@ def _stage_ms(spacings, stage, arith):
 
 
 @pytest.mark.parametrize("arith", ["exact", "fast"])
-@pytest.mark.parametrize("stage", ["density_low"])
+@pytest.mark.parametrize("stage", ["density_low", "force_low"])
 def test_time_grows_with_the_pairs(stage, arith):
     assert _stage_ms(3.0, stage, arith) < 2 * 2.25 * _stage_ms(2.0, stage, arith)

@@ -87,9 +87,10 @@ using namespace gather_detail;
 // states, cutoff d < r and d != 0 against d <= r, the same lambda masks), so
 // testing each listed candidate again with the force's test gives the force's
 // candidates in the same order -- the same sums, bit for bit -- without scanning
-// the ~36 candidates of the window, of which about a third are accepted.  A
-// particle with more than kMaxNbr neighbours, or one whose offset does not fit
-// 16 bits, is marked and walks its window.
+// the ~36 candidates of the window, of which about a third are accepted.  A particle
+// with more than kMaxNbr neighbours is marked kNbrCrowd: its list holds the first of
+// them, and the force walks its window from the last one listed.  One with an offset that
+// does not fit 16 bits is marked kNbrOverflow and walks its whole window.
 //
 // The density pass takes a particle's same-scale window in two phases.  The first
 // walks the window and only tests: it leaves the accepted candidates' offsets in
@@ -159,11 +160,11 @@ __device__ __forceinline__ int nbr_search(const int* off, int dimx, int csx, int
 
 // The rest of a window that holds more than a list: adds the terms of the n entries in
 // the column, searches on from candidate k of row cy until the column is full again, and
-// so on, so that a warp's lanes evaluate their pairs together here too.  Returns false
-// when it comes to a row that does not fit 16 bits.  With a support of 3 lattice spacings
+// so on, so that a warp's lanes evaluate their pairs together here too; its first kMaxNbr
+// neighbours go to the list.  Returns false when it comes to a row that does not fit 16 bits.  With a support of 3 lattice spacings
 // (28 neighbours, 81 candidates) the exact low-res density of 700,000 particles takes 123
-// us, of 4 spacings (50, 144) 156 us; a walk that evaluates at once took 125 and 203 us,
-// and after a search that gave up 320 and 430 us.
+// us without the list and 135 with it, of 4 spacings (50, 144) 156 and 168 us; a walk that
+// evaluates at once took 125 and 203 us, and after a search that gave up 320 and 430 us.
 template <class A, class Key>
 __device__ __forceinline__ bool nbr_crowd(const Params& P, const ScaleView& S, const int* off, int dimx, int csx,
                                           int cex, int cy, int cey, int k, int i, float2 p, float T, int16_t* col,
@@ -172,8 +173,13 @@ __device__ __forceinline__ bool nbr_crowd(const Params& P, const ScaleView& S, c
     int16_t* c = col + n * kNbrCols;
     int b = off[cy * dimx + cex + 1];
     bool fit = true, done = false;
+    int m = 0;
     while (!done) {
-        for (const int16_t* q = col; q < c; q += kNbrCols) sum += A::density(P, sq(sub(p, S.pos[i + *q])));
+        for (const int16_t* q = col; q < c; q += kNbrCols) {
+            const int d = *q;
+            sum += A::density(P, sq(sub(p, S.pos[i + d])));
+            if (d != 0 && m < kMaxNbr) S.nbr[m++ * S.nbr_stride + i] = static_cast<int16_t>(d);
+        }
         c = col;
         done = !fit || cy > cey;
         while (fit && cy <= cey && c <= full) {
@@ -242,7 +248,7 @@ __device__ __forceinline__ void nbr_density(const Params& P, const ScaleView& S,
             ++m;
         }
     }
-    S.nnbr[i] = m <= kMaxNbr ? static_cast<uint8_t>(m) : kNbrOverflow;
+    S.nnbr[i] = m <= kMaxNbr ? static_cast<uint8_t>(m) : kNbrCrowd;
 }
 
 // A same-scale neighbour's state as the force pass reads it.
@@ -268,15 +274,20 @@ __device__ __forceinline__ NbrState fetch_nbr(const ScaleView& S, int k) { retur
 //
 // A group of lanes takes an entry per lane, up to three rounds of entries loaded
 // first.
+//
+// walk(on, from) takes the window's candidates from index `from` on: all of them without
+// a list, those after the first kMaxNbr - 1 neighbours in a crowd.  With a support of 3
+// lattice spacings (28 neighbours) the exact low-res force of 700,000 particles takes 182
+// us, against 324 where the whole window is walked; of 4 spacings (50) 371 and 442 us.
 template <class G, class T, class Test, class Term, class Add, class Walk>
 __device__ __forceinline__ void list_or_walk(bool on, const ScaleView& S, int i, Test&& test, Term&& term, Add&& add,
                                              T& sum, Walk&& walk) {
-    const int nc = S.nnbr[i];
-    const bool listed = nc != kNbrOverflow;
+    const auto listed = [](int mark) { return mark <= kMaxNbr ? mark : (mark == kNbrCrowd ? kMaxNbr - 1 : 0); };
+    const int nc = listed(S.nnbr[i]);
     const int16_t* src = S.nbr + i;
     if constexpr (G::kLanes > 1) {
         constexpr int kRounds = (kMaxNbr + G::kLanes - 1) / G::kLanes;
-        const int m = on && listed ? nc : 0;
+        const int m = on ? nc : 0;
         int dj[kRounds];
 #pragma unroll
         for (int r = 0; r < kRounds; ++r) {
@@ -292,28 +303,31 @@ __device__ __forceinline__ void list_or_walk(bool on, const ScaleView& S, int i,
             if (ok) t = term(n0);
             G::add_lanes(G::ballot(ok), t, add, sum);
         }
-        if (G::any(on && !listed)) walk(on && !listed);
     } else {
-        if (listed) {
-            int d0 = 0, d1 = 0;
-            const auto next = [&](int c) {
-                if (c < nc) d0 = *src;
-                src += S.nbr_stride;
-                d1 = 0;
-                if (c + 1 < nc) d1 = *src;
-                src += S.nbr_stride;
-            };
-            next(0);
-            for (int c = 0; c < nc; c += 2) {
-                const NbrState n0 = fetch_nbr(S, i + d0), n1 = fetch_nbr(S, i + d1);
-                next(c + 2);
-                if (test(n0)) add(sum, term(n0));
-                if (test(n1)) add(sum, term(n1));
-            }
-        } else {
-            walk(true);
+        int d0 = 0, d1 = 0;
+        const auto next = [&](int c) {
+            if (c < nc) d0 = *src;
+            src += S.nbr_stride;
+            d1 = 0;
+            if (c + 1 < nc) d1 = *src;
+            src += S.nbr_stride;
+        };
+        next(0);
+        for (int c = 0; c < nc; c += 2) {
+            const NbrState n0 = fetch_nbr(S, i + d0), n1 = fetch_nbr(S, i + d1);
+            next(c + 2);
+            if (test(n0)) add(sum, term(n0));
+            if (test(n1)) add(sum, term(n1));
         }
     }
+    // the mark is loaded again (the index is hidden, or the compiler would keep it): one
+    // register less in the list loop, without which the tolerance arithmetic's forces took
+    // 4 % longer
+    int again = i;
+    asm("" : "+r"(again));
+    const int mark = S.nnbr[again];
+    if (G::any(on && mark > kMaxNbr))
+        walk(on && mark > kMaxNbr, mark == kNbrCrowd ? i + S.nbr[(kMaxNbr - 1) * S.nbr_stride + i] : 0);
 }
 
 // A particle's same-scale density sum over its window (candidates k with key(k) <= T),
@@ -346,7 +360,7 @@ __device__ __forceinline__ void same_scale_density(bool on, const Params& P, con
                 G::add_lanes(m, ok ? A::density(P, x) : 0.0f, add_density, sum);
             }
         }
-        if (on && G::leader()) S.nnbr[i] = n <= kMaxNbr && fit ? static_cast<uint8_t>(n) : kNbrOverflow;
+        if (on && G::leader()) S.nnbr[i] = fit ? (n <= kMaxNbr ? static_cast<uint8_t>(n) : kNbrCrowd) : kNbrOverflow;
     } else {
         int cy = csy, at = 0;
         // the lanes leave the search at different candidates; without a barrier here those
@@ -358,8 +372,9 @@ __device__ __forceinline__ void same_scale_density(bool on, const Params& P, con
             nbr_density<A>(P, S, i, p, n, nbr_col, sum);
             return;
         }
-        S.nnbr[i] = kNbrOverflow;
+        S.nnbr[i] = kNbrCrowd;
         if (n == kNbrFar || !nbr_crowd<A>(P, S, off, dimx, csx, cex, cy, cey, at, i, p, T, nbr_col, -n, sum, key)) {
+            S.nnbr[i] = kNbrOverflow;
             float x = 0.0f;
             sum = 0.0f;
             G::window(
@@ -670,10 +685,10 @@ __device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V
         const auto term_n = [&](const NbrState& n) {
             return A::template pair<kHLow>(P, pij, x, sub(v, vel_of(n.vq)), qi, n.vq.z, dens, n.vq.w);
         };
-        list_or_walk<G>(valid, L, i, test_n, term_n, add_terms, fl, [&](bool on) {
+        list_or_walk<G>(valid, L, i, test_n, term_n, add_terms, fl, [&](bool on, int from) {
             grid_coord_s<0>(P, p.x, p.y, -P.r, csx, csy);
             grid_coord_s<0>(P, p.x, p.y, P.r, cex, cey);
-            G::window(on, L.off + P.cbL, P.dimL[0], csx, cex, csy, cey, test, term, add_terms, fl);
+            G::window(on, L.off + P.cbL, P.dimL[0], csx, cex, csy, cey, test, term, add_terms, fl, from);
         });
     }
     const int cell = cell_hash_s<0>(P, p);
@@ -836,10 +851,10 @@ __device__ __forceinline__ void force_high_one(const Params& P, const StepView& 
         const auto term_n = [&](const NbrState& n) {
             return A::template pair<kHHigh>(P, pij, x, sub(v, vel_of(n.vq)), qi, n.vq.z, dens, n.vq.w);
         };
-        list_or_walk<G>(valid, H, i, test_n, term_n, add_terms, fh, [&](bool on) {
+        list_or_walk<G>(valid, H, i, test_n, term_n, add_terms, fh, [&](bool on, int from) {
             grid_coord_s<1>(P, p.x, p.y, -P.rh, csx, csy);
             grid_coord_s<1>(P, p.x, p.y, P.rh, cex, cey);
-            G::window(on, H.off + P.cbH, P.dimH[0], csx, cex, csy, cey, test, term, add_terms, fh);
+            G::window(on, H.off + P.cbH, P.dimH[0], csx, cex, csy, cey, test, term, add_terms, fh, from);
         });
     }
     const float2 accB = wall_term<A, G, 1>(valid, P, V, H, i, p, cell_hash_s<0>(P, p));

@@ -27,9 +27,9 @@ struct ScaleView {
     // Neighbour lists the density pass records for the force pass of the same scale:
     // entry c of sorted particle i is
     // nbr[c * nbr_stride + i] = j - i for its c-th same-scale neighbour within the
-    // density's support (itself left out), in window order; nnbr[i] is their count,
-    // kNbrOverflow when there are more than kMaxNbr or an offset does not fit 16
-    // bits.
+    // density's support (itself left out), in window order; nnbr[i] is their count;
+    // kNbrCrowd when there are more than kMaxNbr (the first kMaxNbr are listed); or
+    // kNbrOverflow when an offset does not fit 16 bits (none are).
     int16_t* nbr;
     uint8_t* nnbr;
     long long nbr_stride;  // entries per list column: the scale's capacity
@@ -75,7 +75,7 @@ struct StepView {
 // (82 and 138 us; 28: 78 and 133).  24 is what fits without the handle's memory
 // growing: a grid build borrows the lists for its permutation (12 bytes an entry).
 constexpr int kMaxNbr = 24;
-constexpr uint8_t kNbrOverflow = 255;
+constexpr uint8_t kNbrOverflow = 255, kNbrCrowd = 254;
 
 // Short lists: one particle per thread leaves most of the GPU idle and a step waits
 // for each thread's chain of loads and pairs.  A list of at most so many particles is
