@@ -117,18 +117,18 @@ struct PerGroup {
     template <class T, class Live, class Test, class Term, class Add>
     __device__ __forceinline__ static void window_if(bool on, const int* off, int dimx, int csx, int cex, int csy,
                                                      int cey, Live&& live, Test&& test, Term&& term, Add&& add,
-                                                     T& sum, int from = 0) {
+                                                     T& sum) {
         for (int cy = csy; any(on && cy <= cey); ++cy) {
             const int row = cy * dimx;
             const bool in = on && cy <= cey && live(row);
-            if (any(in)) span(in ? max(off[row + csx], from) : 0, in ? off[row + cex + 1] : 0, test, term, add, sum);
+            if (any(in)) span(in ? off[row + csx] : 0, in ? off[row + cex + 1] : 0, test, term, add, sum);
         }
     }
 
     template <class T, class Test, class Term, class Add>
     __device__ __forceinline__ static void window(bool on, const int* off, int dimx, int csx, int cex, int csy, int cey,
-                                                  Test&& test, Term&& term, Add&& add, T& sum, int from = 0) {
-        window_if(on, off, dimx, csx, cex, csy, cey, [](int) { return true; }, test, term, add, sum, from);
+                                                  Test&& test, Term&& term, Add&& add, T& sum) {
+        window_if(on, off, dimx, csx, cex, csy, cey, [](int) { return true; }, test, term, add, sum);
     }
 };
 

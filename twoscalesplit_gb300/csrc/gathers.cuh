@@ -276,18 +276,19 @@ __device__ __forceinline__ NbrState fetch_nbr(const ScaleView& S, int k) { retur
 // first.
 //
 // walk(on, from) takes the window's candidates from index `from` on: all of them without
-// a list, those after the first kMaxNbr - 1 neighbours in a crowd.  With a support of 3
+// a list, those after the first kMaxNbr - 1 neighbours in a crowd (a group of lanes walks
+// the whole window, 43 us a step of 5,000 such particles; the lists' part of a crowd put
+// 1 % on the steps of short lists without one).  With a support of 3
 // lattice spacings (28 neighbours) the exact low-res force of 700,000 particles takes 182
 // us, against 324 where the whole window is walked; of 4 spacings (50) 371 and 442 us.
 template <class G, class T, class Test, class Term, class Add, class Walk>
 __device__ __forceinline__ void list_or_walk(bool on, const ScaleView& S, int i, Test&& test, Term&& term, Add&& add,
                                              T& sum, Walk&& walk) {
-    const auto listed = [](int mark) { return mark <= kMaxNbr ? mark : (mark == kNbrCrowd ? kMaxNbr - 1 : 0); };
-    const int nc = listed(S.nnbr[i]);
+    int mark = S.nnbr[i];
     const int16_t* src = S.nbr + i;
     if constexpr (G::kLanes > 1) {
         constexpr int kRounds = (kMaxNbr + G::kLanes - 1) / G::kLanes;
-        const int m = on ? nc : 0;
+        const int m = on && mark <= kMaxNbr ? mark : 0;
         int dj[kRounds];
 #pragma unroll
         for (int r = 0; r < kRounds; ++r) {
@@ -303,7 +304,9 @@ __device__ __forceinline__ void list_or_walk(bool on, const ScaleView& S, int i,
             if (ok) t = term(n0);
             G::add_lanes(G::ballot(ok), t, add, sum);
         }
+        if (G::any(on && mark > kMaxNbr)) walk(on && mark > kMaxNbr);
     } else {
+        const int nc = mark <= kMaxNbr ? mark : (mark == kNbrCrowd ? kMaxNbr - 1 : 0);
         int d0 = 0, d1 = 0;
         const auto next = [&](int c) {
             if (c < nc) d0 = *src;
@@ -319,15 +322,14 @@ __device__ __forceinline__ void list_or_walk(bool on, const ScaleView& S, int i,
             if (test(n0)) add(sum, term(n0));
             if (test(n1)) add(sum, term(n1));
         }
+        // the mark is loaded again (the index is hidden, or the compiler would keep it): one
+        // register less in the list loop, without which the tolerance arithmetic's forces
+        // took 4 % longer
+        int again = i;
+        asm("" : "+r"(again));
+        mark = S.nnbr[again];
+        if (mark > kMaxNbr) walk(true, mark == kNbrCrowd ? i + S.nbr[(kMaxNbr - 1) * S.nbr_stride + i] : 0);
     }
-    // the mark is loaded again (the index is hidden, or the compiler would keep it): one
-    // register less in the list loop, without which the tolerance arithmetic's forces took
-    // 4 % longer
-    int again = i;
-    asm("" : "+r"(again));
-    const int mark = S.nnbr[again];
-    if (G::any(on && mark > kMaxNbr))
-        walk(on && mark > kMaxNbr, mark == kNbrCrowd ? i + S.nbr[(kMaxNbr - 1) * S.nbr_stride + i] : 0);
 }
 
 // A particle's same-scale density sum over its window (candidates k with key(k) <= T),
@@ -685,10 +687,10 @@ __device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V
         const auto term_n = [&](const NbrState& n) {
             return A::template pair<kHLow>(P, pij, x, sub(v, vel_of(n.vq)), qi, n.vq.z, dens, n.vq.w);
         };
-        list_or_walk<G>(valid, L, i, test_n, term_n, add_terms, fl, [&](bool on, int from) {
+        list_or_walk<G>(valid, L, i, test_n, term_n, add_terms, fl, [&](bool on, auto... from) {
             grid_coord_s<0>(P, p.x, p.y, -P.r, csx, csy);
             grid_coord_s<0>(P, p.x, p.y, P.r, cex, cey);
-            G::window(on, L.off + P.cbL, P.dimL[0], csx, cex, csy, cey, test, term, add_terms, fl, from);
+            G::window(on, L.off + P.cbL, P.dimL[0], csx, cex, csy, cey, test, term, add_terms, fl, from...);
         });
     }
     const int cell = cell_hash_s<0>(P, p);
@@ -851,10 +853,10 @@ __device__ __forceinline__ void force_high_one(const Params& P, const StepView& 
         const auto term_n = [&](const NbrState& n) {
             return A::template pair<kHHigh>(P, pij, x, sub(v, vel_of(n.vq)), qi, n.vq.z, dens, n.vq.w);
         };
-        list_or_walk<G>(valid, H, i, test_n, term_n, add_terms, fh, [&](bool on, int from) {
+        list_or_walk<G>(valid, H, i, test_n, term_n, add_terms, fh, [&](bool on, auto... from) {
             grid_coord_s<1>(P, p.x, p.y, -P.rh, csx, csy);
             grid_coord_s<1>(P, p.x, p.y, P.rh, cex, cey);
-            G::window(on, H.off + P.cbH, P.dimH[0], csx, cex, csy, cey, test, term, add_terms, fh, from);
+            G::window(on, H.off + P.cbH, P.dimH[0], csx, cex, csy, cey, test, term, add_terms, fh, from...);
         });
     }
     const float2 accB = wall_term<A, G, 1>(valid, P, V, H, i, p, cell_hash_s<0>(P, p));
