@@ -521,8 +521,15 @@ cudaError_t grid_keys_enqueue(const float2* pos, int* n_ptr, int cap, float ox, 
     // on the same tile sums: without them 1.3M points take 13 us instead of 29, and the
     // sums are read off the counts in a kernel of 4 us (the whole build 59 -> 45 us; at
     // 200,000 points 23.5 -> 21 us, at 20,000 no faster).  The steps' key passes hide them
-    // in the force kernels: there, the extra kernel costs 3 us of 360.
-    const bool apart = cap >= kUnrollMin;
+    // in the force kernels: there, the extra kernel costs 3 us of 360.  That kernel reads
+    // every count, so on a grid of many cells a point it costs more than the atomics, from 3
+    // cells a point on for points in cell order and from 28 on for random ones:
+    // whole builds of 150,000 points without / with it, points in cell order and in random
+    // order, on 1.0M cells 27 / 30 and 43 / 29 us, 2.1M 28 / 30 and 39 / 34, 4.2M 31 / 32
+    // and 39 / 38, 16.8M 68 / 75 and 68 / 79, 67M 317 / 370 and 320 / 373; of 1.3M points on
+    // 2.1M cells 44 / 42 and 145 / 60, 8.4M 61 / 64 and 111 / 85, 16.8M 88 / 96 and 124 / 116,
+    // 67M 374 / 423 and 410 / 444.
+    const bool apart = cap >= kUnrollMin && g.ncells / 16 <= cap;
     k_grid_keys<<<particle_blocks(cap, T), T, 0, stream>>>(pos, n_ptr, n_set, ox, oy, cell, dimx, dimy, g.count, g.key,
                                                            g.rank, apart ? nullptr : g.tile_sum);
     cudaError_t e = cudaGetLastError();
