@@ -227,6 +227,7 @@ __global__ void k_grid_scatter(const int* __restrict__ n_ptr, const int32_t* __r
     if (blockIdx.x == 0 && threadIdx.x == 0) {  // the scan's list of big cells, for the reorder
         *g.nbig_snap = *g.nbig;
         *g.nbig = 0;  // empty for the next build's scan
+        *g.by_slot = n < kUnrollMin;
     }
     with_unroll(n, [&](auto unroll) {
         constexpr int U = decltype(unroll)::value;
@@ -254,7 +255,7 @@ __global__ void k_grid_scatter(const int* __restrict__ n_ptr, const int32_t* __r
                     continue;
                 }
                 g.perm[dst] = make_int2(i, d[u]);
-                g.place[dst] = k <= kBigCell ? (k << 8) | (r[u] & 255) : -1;
+                (U == 1 ? g.place[dst] : g.rank[i]) = k <= kBigCell ? (k << 8) | (r[u] & 255) : -1;
             }
         }
     });
@@ -405,21 +406,27 @@ __global__ void __launch_bounds__(kReorderThreads) k_grid_reorder(int* n_ptr, in
                                                                   unsigned* err) {
     wait_for_previous();
     const int n = *g.total;
+    const bool by_slot = *g.by_slot != 0;
     if (blockIdx.x == 0 && threadIdx.x == 0) *n_ptr = n;
     // the tile sums, zero for the next key pass
     const int tiles = ((g.used ? min(*g.used, g.ncells) : g.ncells) + kScanTile - 1) / kScanTile;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < tiles; t += gridDim.x * blockDim.x) g.tile_sum[t] = 0u;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const int2 pe = g.perm[k];
-        const int w = g.place[k];
+        int w = by_slot ? g.place[k] : 0;
         const int src = pe.x, id = pe.y;
-        if (w < 0) continue;  // a big cell's: placed below
-        const int s = k - (w & 255), e = s + (w >> 8);
-        if (src < 0 || src >= cap || s < 0 || e > n || k >= e) {
+        if (src < 0 || src >= cap) {
             atomicOr(err, kErrGridIndex);
             continue;
         }
+        if (!by_slot) w = g.rank[src];
+        if (w < 0) continue;  // a big cell's: placed below
         const Moved m = reorder_load(a, src);  // in flight while the cell's ids are counted
+        const int s = k - (w & 255), e = s + (w >> 8);
+        if (s < 0 || e > n || k >= e) {
+            atomicOr(err, kErrGridIndex);
+            continue;
+        }
         int r = 0;
         for (int j = s; j < e; ++j) r += g.perm[j].y < id;
         reorder_store(a, m, src, s + r, id, err);
@@ -437,7 +444,7 @@ __global__ void __launch_bounds__(kReorderThreads) k_grid_reorder(int* n_ptr, in
             continue;
         }
         const int k = e - s;
-        const int* sorted = block_sort_ids(g.perm + s, k, g.rank + s, g.key + s);
+        const int* sorted = block_sort_ids(g.perm + s, k, (by_slot ? g.rank : g.place) + s, g.key + s);
         __syncthreads();
         for (int j = threadIdx.x; j < k; j += blockDim.x) {
             const int2 pe = g.perm[s + j];
@@ -483,9 +490,10 @@ GridBufs grid_bufs_carve(void* base, int cap, int ncells, bool own_off, bool own
     g.tile_sum = reinterpret_cast<unsigned*>(p);
     p += al(sizeof(unsigned) * (size_t)g.ntiles);
     g.used = nullptr;
-    g.total = reinterpret_cast<int*>(p);  // 256 bytes: total, nbig, nbig_snap
+    g.total = reinterpret_cast<int*>(p);  // 256 bytes: total, nbig, nbig_snap, by_slot
     g.nbig = g.total + 1;
     g.nbig_snap = g.total + 2;
+    g.by_slot = g.total + 3;
     p += 256;
     g.off = nullptr;
     if (own_off) {
