@@ -15,7 +15,7 @@ BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libtss.so")
 SOURCES = ["grid.cu", "grid_noalloc.cu", "sph.cu", "sph_fast.cu", "solver.cu", "pool.cu", "render.cu", "serve.cpp"]
 HEADERS = ["tss_device.cuh", "arith.cuh", "gather.cuh", "gathers.cuh", "grid.cuh", "sph.cuh", "solver_impl.cuh",
-           "extent.hpp"]
+           "extent.hpp", "trips.hpp"]
 ARCH = os.environ.get("TSS_CUDA_ARCH", "103a")
 
 

@@ -7,6 +7,7 @@
 
 #include "../../include/tss.h"
 #include "grid.cuh"
+#include "trips.hpp"
 
 namespace tss {
 
@@ -49,19 +50,19 @@ __global__ void k_grid_keys(const float2* __restrict__ pos, int* n_ptr, int n_se
     if (n_set >= 0 && blockIdx.x == 0 && threadIdx.x == 0) *n_ptr = n_set;
     with_unroll(n, [&](auto unroll) {
         constexpr int U = decltype(unroll)::value;
-        for (int base = blockIdx.x * blockDim.x * U; base < n; base += gridDim.x * blockDim.x * U) {
+        for_trips<U>(n, blockIdx.x, gridDim.x, threadIdx.x, blockDim.x, [&](unsigned base) {
             int c[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const int i = base + u * blockDim.x + threadIdx.x;
-                c[u] = i < n ? cell_hash(pos[i], ox, oy, cell, dimx, dimy) : -1;
+                const unsigned i = base + u * blockDim.x;
+                c[u] = i < static_cast<unsigned>(n) ? cell_hash(pos[i], ox, oy, cell, dimx, dimy) : -1;
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const int i = base + u * blockDim.x + threadIdx.x;
-                if (c[u] >= 0) grid_key(count, key, rank, tile_sum, i, c[u]);
+                const unsigned i = base + u * blockDim.x;
+                if (c[u] >= 0) grid_key(count, key, rank, tile_sum, static_cast<int>(i), c[u]);
             }
-        }
+        });
     });
 }
 
@@ -231,18 +232,19 @@ __global__ void k_grid_scatter(const int* __restrict__ n_ptr, const int32_t* __r
     }
     with_unroll(n, [&](auto unroll) {
         constexpr int U = decltype(unroll)::value;
-        for (int base = blockIdx.x * blockDim.x * U; base < n; base += gridDim.x * blockDim.x * U) {
+        for_trips<U>(n, blockIdx.x, gridDim.x, threadIdx.x, blockDim.x, [&](unsigned base) {
             int c[U], r[U], d[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const int i = base + u * blockDim.x + threadIdx.x;
-                c[u] = i < n ? g.key[i] : -1;  // negative: dropped from the list
-                r[u] = i < n ? g.rank[i] : 0;
-                d[u] = i < n ? id[i] : 0;
+                const unsigned i = base + u * blockDim.x;
+                const bool in = i < static_cast<unsigned>(n);
+                c[u] = in ? g.key[i] : -1;  // negative: dropped from the list
+                r[u] = in ? g.rank[i] : 0;
+                d[u] = in ? id[i] : 0;
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const int i = base + u * blockDim.x + threadIdx.x;
+                const int i = static_cast<int>(base + u * blockDim.x);
                 if (c[u] < 0) continue;
                 if (c[u] >= g.ncells) {
                     atomicOr(err, kErrGridIndex);
@@ -257,7 +259,7 @@ __global__ void k_grid_scatter(const int* __restrict__ n_ptr, const int32_t* __r
                 g.perm[dst] = make_int2(i, d[u]);
                 (U == 1 ? g.place[dst] : g.rank[i]) = k <= kBigCell ? (k << 8) | (r[u] & 255) : -1;
             }
-        }
+        });
     });
 }
 
@@ -411,26 +413,28 @@ __global__ void __launch_bounds__(kReorderThreads) k_grid_reorder(int* n_ptr, in
     // the tile sums, zero for the next key pass
     const int tiles = ((g.used ? min(*g.used, g.ncells) : g.ncells) + kScanTile - 1) / kScanTile;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < tiles; t += gridDim.x * blockDim.x) g.tile_sum[t] = 0u;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    for_trips<1>(n, blockIdx.x, gridDim.x, threadIdx.x, blockDim.x, [&](unsigned slot) {
+        if (slot >= static_cast<unsigned>(n)) return;
+        const int k = static_cast<int>(slot);
         const int2 pe = g.perm[k];
         int w = by_slot ? g.place[k] : 0;
         const int src = pe.x, id = pe.y;
         if (src < 0 || src >= cap) {
             atomicOr(err, kErrGridIndex);
-            continue;
+            return;
         }
         if (!by_slot) w = g.rank[src];
-        if (w < 0) continue;  // a big cell's: placed below
+        if (w < 0) return;  // a big cell's: placed below
         const Moved m = reorder_load(a, src);  // in flight while the cell's ids are counted
         const int s = k - (w & 255), e = s + (w >> 8);
         if (s < 0 || e > n || k >= e) {
             atomicOr(err, kErrGridIndex);
-            continue;
+            return;
         }
         int r = 0;
         for (int j = s; j < e; ++j) r += g.perm[j].y < id;
         reorder_store(a, m, src, s + r, id, err);
-    }
+    });
     const int nb = min(*g.nbig_snap, g.big_cap);
     for (int b = blockIdx.x; b < nb; b += gridDim.x) {
         const int c = g.big[b];
