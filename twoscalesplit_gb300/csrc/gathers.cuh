@@ -9,11 +9,11 @@
 // contiguous span [off[row + cx0], off[row + cx1 + 1]).  Each particle's sums take
 // its candidates in the reference's order (cells row by row, particles in cell
 // order), which keeps every FP32 sum identical to the reference's for the same
-// list order.  The gathers walk a particle's window one of two ways (gather.cuh):
-// one particle per thread, consecutive threads walking overlapping spans so that
-// neighbour loads are shared through L1 (the throughput form), or one particle per
-// warp with the candidates spread over the lanes (for scenes too small to fill the
-// GPU); both give the same bits.
+// list order.  A particle is taken in one of three ways (gather.cuh): by one thread,
+// consecutive threads with overlapping windows so that neighbour loads are shared
+// through L1 (the throughput form); by a group of 8 or 4 lanes, where a list is too
+// short to fill the GPU that way (by_size); or by a warp, a launch shape of its own.
+// All give the same bits.
 //
 // Each kernel's per-particle work is an inlined function of the particle's Params:
 // the kernel's own constants for a single scene, the scene's table row for a
@@ -80,9 +80,8 @@ __device__ __forceinline__ void by_size(int n, F&& f) {
 }  // namespace gather_detail
 using namespace gather_detail;
 
-// Neighbour lists (ScaleView::nbr).  A density pass that runs one particle per
-// thread records the same-scale candidates its window accepts, in window order,
-// and the force pass of the same step walks that list instead of its window: the
+// Neighbour lists (ScaleView::nbr).  The density pass records the same-scale
+// candidates that a particle's window accepts, in window order, and the force pass of the same step walks that list instead of its window: the
 // force's own candidates are a subset of the density's (same positions and
 // states, cutoff d < r and d != 0 against d <= r, the same lambda masks), so
 // testing each listed candidate again with the force's test gives the force's
@@ -776,12 +775,13 @@ __device__ __forceinline__ bool force_low_one(const Params& P, const StepView& V
 // A warp-uniform loop (every lane makes the same number of trips, lanes past n
 // inactive) so the ballot that feeds the split compaction sees whole warps; a warp's
 // particles lie in one compaction tile (kSplitTile % 32 == 0).
-// 48 registers (five blocks per SM) in both forms of the exact arithmetic.  The
-// batched form measured the same at 40 and 48 on a batch of 512 mixed scenes (4.11
-// / 4.08 ms), 3-7 % faster at 48 on batches of one scene, and 10 % slower at 64.
-// The single-scene form in the tolerance arithmetic fits 40 registers without
-// spilling and runs six blocks per SM: 3.5 % faster on the developed 1M dam break
-// (0.130 -> 0.125 ms); batched, it would spill 76 bytes at 40 and keeps 48.
+// 48 registers (five blocks per SM) in both forms of the exact arithmetic, 40 (six) in
+// the tolerance arithmetic's single-scene form; one block per SM more or fewer was slower.
+// The kernel holds the forms for short lists too
+// (by_size), and they share the register bound with the long lists' form: it spills 124 /
+// 160 bytes (stores / loads) in the exact arithmetic and 88 / 140 in the tolerance one,
+// batched 420 / 680 and 164 / 164; without the short forms it would be 48 / 48, 16 / 16,
+// 220 / 204 and 36 / 40.
 template <bool B, class G, class A>
 __global__ void __launch_bounds__(256, (A::kFast && !B) ? 6 : 5) k_force_low(Params P0, StepView V) {
     let_next_start();
@@ -949,17 +949,14 @@ __device__ __forceinline__ void force_high_one(const Params& P, const StepView& 
     }
 }
 
-// Register budgets measured per form.  The batched form reads each particle's
-// parameters from the scene table: at 40 registers it spilled ~300 bytes, at 48 a
-// third of that, at 64 (four blocks per SM) nothing -- as fast as 48 on a batch of
-// 512 mixed scenes and 15 % faster on a batch of one 162k-particle scene.  The
-// single-scene form at 48 registers (five blocks) spills 64 bytes instead of 120
-// at 40 and measured 3-4 % faster.  In the tolerance arithmetic the single-scene
-// form needs no spill at 40 registers (six blocks per SM) and is 3.8 % faster there
-// on the developed 1M dam break (0.159 -> 0.153 ms).  The batched form in the
-// tolerance arithmetic runs five blocks per SM (48 registers, 28 bytes spilled):
-// 4 % faster than four on the 512-scene batch (2.16 against 2.26 ms), where the
-// exact arithmetic's batched form was 8 % slower at five.
+// Registers: 48 (five blocks per SM) in the exact arithmetic's single-scene form and the
+// tolerance arithmetic's batched one, 40 (six) and 64 (four) in the other two.  On a dam
+// break of 1.0M + 1.0M particles five blocks took 130 us and four 140 (exact), six 86 and
+// five 90.5 (tolerance), and one more was slower too.  The batched form reads
+// each particle's parameters from the scene table, which is what its registers go to.
+// Spills, with the forms for short lists in the same kernel (see k_force_low): 240 / 356
+// bytes exact, 128 / 212 in the tolerance arithmetic, batched 40 / 116 and 188 / 224;
+// without the short forms 80 / 92, 8 / 8, 28 / 32 and 52 / 56.
 template <bool B, class G, class A>
 __global__ void __launch_bounds__(256, B ? (A::kFast ? 5 : 4) : (A::kFast ? 6 : 5)) k_force_high(Params P0, StepView V) {
     by_size<G, true>(V.cnt->cur[1], [&](auto form, int n) {

@@ -36,8 +36,8 @@
 namespace tss {
 
 // The scatter and the reorder wait for chains of dependent loads (a fifth of the copy
-// rate at 1.0M entries).  With four of the scatter's entries in flight per thread, and
-// the reorder going from the permutation to the cell's ids without the key and the
+// rate at 1.0M entries).  With four of the key pass's and the scatter's entries in flight
+// per thread, and the reorder going from the permutation to the cell's ids without the key and the
 // offsets between (its state loads in flight meanwhile), a build of 1.0M entries in the
 // step took 37 -> 33 us; the step of 1.0M + 1.0M particles 364 -> 359 us, of 5,000
 // (graphs of eight) 31.8 -> 30.5 us.
@@ -120,10 +120,11 @@ __global__ void k_grid_reorder(int* n_ptr, int cap, GridBufs g, ReorderArgs a, u
 // let_next_start() (or ended).  wait_for_previous() returns when the predecessor has
 // ended and its writes are visible; nothing the predecessor writes, or reads and the
 // kernel overwrites, may be touched before it.  Without such a launch both are no-ops.
-// The scatter and the reorder start so (their launches overlap the kernel before), and
-// the high-res force, which takes its own scale's pairs beside the low-res force's last
-// blocks.  With the two clears that stood between these kernels done by kernels instead,
-// a step took 52 -> 39 us at 5,000 particles, 113 -> 91 us at 162,000 (fast launches and
+// Scan, scatter and reorder start so, the kernel that counts the tiles of a build of its
+// own, the relaxation's three kernels (their launches overlap the kernel before), and the
+// high-res force, which takes its own scale's pairs beside the low-res force's last blocks.
+// With the two clears that stood between these kernels done by kernels instead, a step
+// took 52 -> 39 us at 5,000 particles, 113 -> 91 us at 162,000 (fast launches and
 // overlap), 398 -> 379 us at 1.0M + 1.0M.  All other launches of a step the same way: no
 // faster (379 -> 380 us, 91 -> 93 us).
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

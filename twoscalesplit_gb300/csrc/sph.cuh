@@ -57,7 +57,7 @@ struct StepView {
     Counters* cnt;
     uint8_t* split_flag;    // [n_low]
     int32_t* split_ids;     // [n_low] parents split this step (= next step's fresh list)
-    unsigned* split_tile;   // [ceil(n_low / kSplitTile)] splits per tile, zero at step start
+    unsigned* split_tile;   // [ceil(n_low / kSplitTile)] splits per tile: cleared by the low-res density, counted by the force
     float2* relax_pos;      // [capH] relaxation scratch
     float2* relax_vel;
     int nL;                 // low-res count (constant for a solver)
@@ -88,7 +88,10 @@ constexpr uint8_t kNbrOverflow = 255, kNbrCrowd = 254;
 //   low dens.  11 / 11 / 11 / 9   11 / 13 / 11 / 11  12 / 13 / 14 / 17  13 / 17 / 21 / 25
 //   high dens. 12 / 11 / 10 / 8   12 / 12 / 10 / 12  12 / 13 / 14 / 16  17 / 17 / 20 / 26
 // A density search is short and its groups do more work than its threads (the two run
-// as parallel branches), so it returns to one thread earlier than a force does.
+// as parallel branches), so it returns to one thread earlier than a force does.  The limits
+// lie inside that sweep, which has no size between those shown and was taken in the exact
+// arithmetic alone: 8 lanes are still a little ahead of 4 at 22,000, and 4 lanes ahead of
+// one thread at 48,000, its last size.
 constexpr int kDensity8Max = 12000;
 constexpr int kForce8Max = 20000, kForce4Max = 48000;
 
